@@ -21,6 +21,8 @@ splits H x W into overlapping tiles blended with linear feathering.
 """
 from __future__ import annotations
 
+import functools
+
 import torch
 import torch.nn as nn
 import torch.nn.functional as F
@@ -242,35 +244,49 @@ class VideoVAE_(nn.Module):
         self.conv2 = CausalConv3d(z_dim, z_dim, 1)
         self.decoder = Decoder3d(dim, z_dim, dim_mult, num_res_blocks, attn_scales, temperal_downsample[::-1], dropout)
 
-    def encode(self, x, scale, chunk_frames: int = 0):
+    def encode(self, x, scale, chunk_frames: int = 0, run=None):
         """``chunk_frames`` > 0: the first frame, then that many frames at a time (a multiple of 4), with the
-        convolutions' history carried between chunks."""
+        convolutions' history carried between chunks.  ``run``: a ``wan_vae_native.Run`` that may compute this pass."""
+        encoder, first = self.encoder, 1
+        # three stride-2 windows need two pixels each
+        if run is not None and min(x.shape[3], x.shape[4]) >= 16:
+            encoder = functools.partial(run.encoder, self.encoder)
+            first = 1 + chunk_frames                              # frame 0 rides with the first chunk
         if chunk_frames and x.shape[2] > 1:
             assert chunk_frames % 4 == 0 and (x.shape[2] - 1) % 4 == 0, "chunks of 4k frames after the first frame"
             outs = []
             with _streaming(StreamState()):
-                outs.append(self.encoder(x[:, :, :1]))
-                for t0 in range(1, x.shape[2], chunk_frames):
-                    outs.append(self.encoder(x[:, :, t0:t0 + chunk_frames]))
+                outs.append(encoder(x[:, :, :first]))
+                for t0 in range(first, x.shape[2], chunk_frames):
+                    outs.append(encoder(x[:, :, t0:t0 + chunk_frames]))
             h = torch.cat(outs, dim=2)
         else:
-            h = self.encoder(x)
+            h = encoder(x)
         mu, _logvar = self.conv1(h).chunk(2, dim=1)
         mean, inv_std = scale
         return (mu - mean.view(1, -1, 1, 1, 1)) * inv_std.view(1, -1, 1, 1, 1)
 
-    def decode(self, z, scale, chunk_frames: int = 0):
-        """``chunk_frames`` > 0: that many latent frames at a time (the reference decodes one by one)."""
+    def decode(self, z, scale, chunk_frames: int = 0, run=None):
+        """``chunk_frames`` > 0: that many latent frames at a time (the reference decodes one by one).  ``run``: a
+        ``wan_vae_native.Run`` that may compute this pass."""
         mean, inv_std = scale
         z = z / inv_std.view(1, -1, 1, 1, 1) + mean.view(1, -1, 1, 1, 1)
         x = self.conv2(z)
+        decoder = self.decoder if run is None else functools.partial(run.decoder, self.decoder)
         if chunk_frames and x.shape[2] > 1:
             outs = []
             with _streaming(StreamState()):
                 for t0 in range(0, x.shape[2], chunk_frames):
-                    outs.append(self.decoder(x[:, :, t0:t0 + chunk_frames]).clamp_(-1, 1))
+                    outs.append(decoder(x[:, :, t0:t0 + chunk_frames]).clamp_(-1, 1))
             return torch.cat(outs, dim=2)
-        return self.decoder(x).clamp_(-1, 1)
+        return decoder(x).clamp_(-1, 1)
+
+
+def open_run(net, x):
+    """A ``wan_vae_native.Run`` when the native kernels may compute ``net(x)``, else None."""
+    from . import wan_vae_native
+
+    return wan_vae_native.open_run(net, x)
 
 
 class WanVideoVAE(nn.Module):
@@ -352,13 +368,14 @@ class WanVideoVAE(nn.Module):
         for v in videos:
             x = v.unsqueeze(0).to(device or v.device)
             scale = self._scale(x)
-            ck = self._chunk(x.shape[2], chunk_frames, 4)
+            run = open_run(self.model.encoder, x)
+            ck = self._chunk(x.shape[2], chunk_frames, 4 if run is None else 16)
             if tiled:
                 tile = (tile_size[0] * 8, tile_size[1] * 8)
                 stride = (tile_stride[0] * 8, tile_stride[1] * 8)
-                z = self._tiled(lambda t: self.model.encode(t, scale, ck), x, tile, stride, 1 / 8, self.z_dim)
+                z = self._tiled(lambda t: self.model.encode(t, scale, ck, run), x, tile, stride, 1 / 8, self.z_dim)
             else:
-                z = self.model.encode(x, scale, ck)
+                z = self.model.encode(x, scale, ck, run)
             outs.append(z.squeeze(0))
         return torch.stack(outs)
 
@@ -368,10 +385,12 @@ class WanVideoVAE(nn.Module):
         for z in latents:
             z = z.unsqueeze(0).to(device or z.device)
             scale = self._scale(z)
-            ck = self._chunk(4 * (z.shape[2] - 1) + 1, chunk_frames, 1)
+            # bf16 weights are refused by the decoder's enlargement layers, with and without the native kernels
+            run = open_run(self.model.decoder, z) if z.dtype == torch.float32 else None
+            ck = self._chunk(4 * (z.shape[2] - 1) + 1, chunk_frames, 1 if run is None else 4)
             if tiled:
-                v = self._tiled(lambda t: self.model.decode(t, scale, ck), z, tile_size, tile_stride, 8, 3)
+                v = self._tiled(lambda t: self.model.decode(t, scale, ck, run), z, tile_size, tile_stride, 8, 3)
             else:
-                v = self.model.decode(z, scale, ck)
+                v = self.model.decode(z, scale, ck, run)
             outs.append(v.squeeze(0))
         return torch.stack(outs)

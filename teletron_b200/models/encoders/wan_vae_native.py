@@ -1,0 +1,191 @@
+"""The VAE's encoder and decoder on the library's convolution kernels (ops/conv.py), module by module the function
+of ``wan_vae.Encoder3d`` / ``Decoder3d`` (teletron/models/wan/encoder/wan_video_vae.py:34-420 in the reference).
+
+Activations stay in the channel-chunked layout from the first convolution to the last; norm + SiLU write straight into
+the buffer that the following convolution reads, behind the history frames of a chunked pass; the residual is added in
+the convolution's epilogue; temporal up-sampling stores its two channel halves into alternating frames.
+"""
+from __future__ import annotations
+
+import torch
+import torch.nn as nn
+
+from ...ops import conv as C
+from . import wan_vae as V
+
+
+def usable(net: nn.Module, x: torch.Tensor) -> bool:
+    """Whether this forward pass may take the native kernels: one clip on a GPU, bf16 or fp32 with TF32 convolutions
+    allowed (torch's default), weights of the same type, no gradients, hooks or tracing, channel counts in multiples
+    of 16 up to 384 behind the first convolution."""
+    if not (x.is_cuda and x.dim() == 5 and x.shape[0] == 1 and x.numel() > 0):
+        return False
+    if x.dtype == torch.float32:
+        if not (torch.backends.cudnn.enabled and torch.backends.cudnn.allow_tf32):
+            return False
+    elif x.dtype != torch.bfloat16:
+        return False
+    if torch.is_autocast_enabled("cuda") or torch.jit.is_tracing() or torch.compiler.is_compiling():
+        return False
+    if type(x) is not torch.Tensor or torch._C._functorch.is_functorch_wrapped_tensor(x):
+        return False
+    if torch.nn.modules.module._has_any_global_hook():
+        return False
+    grad = torch.is_grad_enabled()
+    if grad and x.requires_grad:
+        return False
+    first, last = net.conv1, net.head[2]
+    for m in net.modules():
+        if m._forward_hooks or m._forward_pre_hooks:
+            return False
+        if isinstance(m, nn.Dropout) and m.training and m.p > 0:
+            return False
+        if isinstance(m, (nn.Conv2d, nn.Conv3d)):
+            if (m.in_channels % 16 and m is not first) or (m.out_channels % 16 and m is not last):
+                return False
+            if m is not first and m.in_channels > 384:
+                return False
+        for p in m._parameters.values():
+            if p is not None and (p.device != x.device or p.dtype != x.dtype or type(p) is not nn.Parameter
+                                  or (grad and p.requires_grad)):
+                return False
+    return True
+
+
+def open_run(net: nn.Module, x: torch.Tensor):
+    return Run() if usable(net, x) else None
+
+
+class Run:
+    """One encode / decode call: the packed weights, shared by its chunks and tiles."""
+
+    def __init__(self):
+        self.packs = {}
+
+    def pack(self, m, kind):
+        pk = self.packs.get(m)
+        if pk is None:
+            pk = self.packs[m] = C.PackedConv(m.weight, m.bias, kind)
+        return pk
+
+    def gamma(self, m):
+        g = self.packs.get(m)
+        if g is None:
+            g = self.packs[m] = m.gamma.detach().float().reshape(-1).contiguous()
+        return g
+
+    # -------------------------------------------------------------------------------------------------- pieces
+    def _with_history(self, m, shape, like):
+        """Buffer for the input of causal convolution ``m`` (two frames of history), the view to fill and the frame
+        offset of its first window."""
+        st = V._STREAM
+        hist = st.get(m) if st is not None else None
+        n = 0 if hist is None else 2
+        buf = torch.empty((shape[0] + n, *shape[1:]), dtype=like.dtype, device=like.device)
+        if n:
+            buf[:2].copy_(hist)
+        return buf, buf[n:], n - 2
+
+    @staticmethod
+    def _keep_history(m, buf):
+        st = V._STREAM
+        if st is not None:
+            tail = buf[-2:].clone()
+            st[m] = tail if tail.shape[0] == 2 else torch.cat([torch.zeros_like(tail), tail])
+
+    def norm_conv(self, norm, m, x, res=None, planar=False):
+        buf, view, t_off = self._with_history(m, x.shape, x)
+        C.chan_norm(x, self.gamma(norm), view)
+        self._keep_history(m, buf)
+        return C.conv(buf, self.pack(m, C.CONV_SPATIAL), x.shape[0], x.shape[2:4], t_off=t_off, res=res, planar=planar)
+
+    def first_conv(self, m, x):
+        """x: planar [C, T, H, W]."""
+        x = C.from_planar(x, round_tf32=True)
+        frames, t_off = x.shape[0], -2
+        st = V._STREAM
+        if st is not None and st.get(m) is not None:
+            x, t_off = torch.cat([st[m], x]), 0
+        self._keep_history(m, x)
+        return C.conv(x, self.pack(m, C.CONV_SPATIAL), frames, x.shape[2:4], t_off=t_off)
+
+    def res_block(self, m, x):
+        r = m.residual
+        h = self.norm_conv(r[0], r[2], x)
+        if isinstance(m.shortcut, nn.Identity):
+            skip = x
+        else:
+            skip = C.conv(C.rounded(x), self.pack(m.shortcut, C.CONV_POINT), x.shape[0], x.shape[2:4])
+        return self.norm_conv(r[3], r[6], h, res=skip)
+
+    def attention(self, m, x):
+        return C.from_planar(m(C.to_planar(x).unsqueeze(0)).squeeze(0))
+
+    def down(self, m, x):
+        st = V._STREAM
+        first = st is None or ("seen", m) not in st
+        if st is not None:
+            st[("seen", m)] = True
+        hw = (x.shape[2] // 2, x.shape[3] // 2)
+        x = C.conv(C.phases2(x), self.pack(m.resample[1], C.CONV_STRIDE2), x.shape[0], hw)
+        if m.mode != "downsample3d":
+            return x
+        last = x[-1:].clone() if st is not None else None
+        t = x.shape[0]
+        if not first:
+            x, t, keep = torch.cat([st[("last", m)], x]), t + 1, 0
+        else:
+            keep = 1
+        if t > 1:
+            n = (t - 3) // 2 + 1
+            out = torch.empty((keep + n, *x.shape[1:]), dtype=x.dtype, device=x.device)
+            if keep:
+                out[0].copy_(x[0])
+            C.conv(C.rounded(x), self.pack(m.time_conv, C.CONV_POINT), n, hw, t_stride=2, out=out[keep:])
+            x = out
+        if st is not None:
+            st[("last", m)] = last
+        return x
+
+    def up(self, m, x):
+        st = V._STREAM
+        first = st is None or ("seen", m) not in st
+        if st is not None:
+            st[("seen", m)] = True
+        t, hw = x.shape[0], x.shape[2:4]
+        if m.mode == "upsample3d":
+            keep = 1 if first else 0
+            if t > keep:
+                rest = x[keep:]
+                buf, view, t_off = self._with_history(m.time_conv, rest.shape, x)
+                C.rounded(rest, out=view)
+                self._keep_history(m.time_conv, buf)
+                out = torch.empty((keep + 2 * (t - keep), *x.shape[1:]), dtype=x.dtype, device=x.device)
+                if keep:
+                    out[0].copy_(x[0])
+                C.conv(buf, self.pack(m.time_conv, C.CONV_POINT), t - keep, hw, t_off=t_off, out=out[keep:], t_mul=2)
+                x = out
+        return C.conv(C.enlarge2(x), self.pack(m.resample[1], C.CONV_SPATIAL), x.shape[0], (2 * hw[0], 2 * hw[1]))
+
+    # ------------------------------------------------------------------------------------------------- networks
+    def _layers(self, layers, x):
+        for m in layers:
+            if isinstance(m, V.ResidualBlock):
+                x = self.res_block(m, x)
+            elif isinstance(m, V.AttentionBlock):
+                x = self.attention(m, x)
+            else:
+                x = self.down(m, x) if m.mode.startswith("down") else self.up(m, x)
+        return x
+
+    def encoder(self, net, x):
+        """[1, 3, T, H, W] -> [1, 2 z, T', H / 8, W / 8], the same as ``net(x)``."""
+        h = self._layers(net.downsamples, self.first_conv(net.conv1, x[0]))
+        h = self._layers(net.middle, h)
+        return self.norm_conv(net.head[0], net.head[2], h, planar=True).unsqueeze(0)
+
+    def decoder(self, net, z):
+        """[1, z, T, H, W] -> [1, 3, T', 8 H, 8 W], the same as ``net(z)``."""
+        h = self._layers(net.middle, self.first_conv(net.conv1, z[0]))
+        h = self._layers(net.upsamples, h)
+        return self.norm_conv(net.head[0], net.head[2], h, planar=True).unsqueeze(0)
