@@ -4,8 +4,8 @@ bidirectional buckets, vocabulary 256384.
 
 Module names follow the reference text encoder (teletron/models/wan/encoder/
 wan_video_text_encoder.py:210-255): ``token_embedding``, ``blocks.N.{norm1, attn.{q,k,v,o}, pos_embedding.
-embedding, norm2, ffn.{gate.0, fc1, fc2}}``, ``norm``.  Plain PyTorch: the encoder runs once per
-sample on dedicated encoder ranks, not on the DiT hot path.
+embedding, norm2, ffn.{gate.0, fc1, fc2}}``, ``norm``.  The encoder runs once per sample on dedicated encoder ranks:
+projections and attention are library calls, what lies between them runs in fused kernels (csrc/t5.cu) on a GPU.
 """
 from __future__ import annotations
 
@@ -14,6 +14,8 @@ import math
 import torch
 import torch.nn as nn
 import torch.nn.functional as F
+
+from ...ops import t5 as t5_ops
 
 
 class T5LayerNorm(nn.Module):
@@ -116,7 +118,53 @@ class UMT5Encoder(nn.Module):
                                      for _ in range(num_layers)])
         self.norm = T5LayerNorm(dim)
 
+    def _native(self, ids, mask):
+        """Whether the fused kernels (csrc/t5.cu) may run: dense bf16 parameters on the ids' GPU, per-layer position
+        tables, a [B, L] mask or none, and nothing that would notice the skipped modules (gradients, hooks, tracing)."""
+        w = self.token_embedding.weight
+        if not (ids.is_cuda and w.dtype == torch.bfloat16 and ids.dim() == 2 and ids.numel() > 0 and ids.shape[1] <= 4096):
+            return False
+        if self.pos_embedding is not None or self.dim % 8 or self.dim > 8192 or len(self.blocks) == 0:
+            return False
+        if mask is not None and (mask.shape != ids.shape or mask.device != ids.device):
+            return False
+        if torch.is_autocast_enabled("cuda") or torch.jit.is_tracing() or torch.compiler.is_compiling():
+            return False
+        if torch.nn.modules.module._has_any_global_hook() or type(ids) is not torch.Tensor:
+            return False
+        if torch._C._functorch.is_functorch_wrapped_tensor(ids):
+            return False
+        grad = torch.is_grad_enabled()
+        for m in self.modules():
+            if m is not self and (m._forward_hooks or m._forward_pre_hooks):
+                return False
+            for p in m._parameters.values():
+                if p is not None and (p.dtype != torch.bfloat16 or p.device != ids.device or not p.is_contiguous()
+                                      or (grad and p.requires_grad) or p.data_ptr() % 16):
+                    return False
+        return self.blocks[0].ffn.fc1.weight.shape[0] % 8 == 0
+
+    def _forward_native(self, ids, mask):
+        b, n = ids.shape
+        x = self.token_embedding(ids)
+        bucket = self.blocks[0].pos_embedding._bucket(torch.arange(1 - n, n, device=ids.device)).int()
+        keep = None if mask is None else (mask != 0).to(torch.uint8).contiguous()
+        norm = self.blocks[0].norm1
+        x, h = t5_ops.add_norm(x, None, norm.weight, norm.eps)
+        for i, blk in enumerate(self.blocks):
+            at = blk.attn
+            q, k, v = (lin(h).view(b, n, at.num_heads, at.head_dim).transpose(1, 2) for lin in (at.q, at.k, at.v))
+            bias = t5_ops.bias(blk.pos_embedding.embedding.weight, bucket, keep, b, at.num_heads, n)
+            o = F.scaled_dot_product_attention(q, k, v, attn_mask=bias, scale=1.0)
+            x, h = t5_ops.add_norm(x, at.o(o.transpose(1, 2).reshape(b, n, -1)), blk.norm2.weight, blk.norm2.eps)
+            f = blk.ffn.fc2(t5_ops.geglu(blk.ffn.fc1(h), blk.ffn.gate[0](h)))
+            norm = self.blocks[i + 1].norm1 if i + 1 < len(self.blocks) else self.norm
+            x, h = t5_ops.add_norm(x, f, norm.weight, norm.eps)
+        return h
+
     def forward(self, ids, mask=None):
+        if self._native(ids, mask):
+            return self._forward_native(ids, mask)
         x = self.token_embedding(ids)
         e = self.pos_embedding(x.shape[1], x.shape[1]) if self.pos_embedding is not None else None
         for blk in self.blocks:
