@@ -243,7 +243,11 @@ TT_API int tt_gemm_bf16(const void* A, long long lda, int a_mn, const void* B, l
     TT_CHECK((((uintptr_t)residual | (uintptr_t)gate) & 15) == 0, "gemm: residual/gate misaligned");
   }
   if (bias) TT_CHECK(((uintptr_t)bias & 15) == 0, "gemm: bias is not 16-byte aligned");
-  const int BN = N > 128 ? 256 : (N > 64 ? 128 : 64);
+  int dev = 0, sms = 0;
+  TT_CUDA(cudaGetDevice(&dev));
+  TT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const int split = (max_ctas <= 0 && N > 64) ? splitk_factor(M, N, K, sms) : 1;
+  const int BN = split > 1 ? 128 : N > 128 ? 256 : (N > 64 ? 128 : 64);
   CUtensorMap tmA, tmB;
   {
     uint64_t dims[2], str[1];
@@ -266,9 +270,7 @@ TT_API int tt_gemm_bf16(const void* A, long long lda, int a_mn, const void* B, l
   p.aux_out = (bf16*)aux_out; p.alpha = alpha; p.status = status;
   p.tp_mode = 0; p.seg_rows = 0; p.world = 1; p.rank = 0;
   for (int i = 0; i < TP_MAX; ++i) p.peer_c[i] = nullptr;
-  int dev = 0, sms = 0;
-  TT_CUDA(cudaGetDevice(&dev));
-  TT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  if (split > 1) return tt_gemm_splitk(tmA, tmB, a_mn, b_mn, p, split, stream);
   if (max_ctas > 0 && max_ctas < sms) sms = max_ctas;
   if (BN == 256) return dispatch_major<256>(a_mn, b_mn, tmA, tmB, p, sms, stream);
   if (BN == 128) return dispatch_major<128>(a_mn, b_mn, tmA, tmB, p, sms, stream);

@@ -70,6 +70,89 @@ __device__ __forceinline__ MTile m_tile(const GemmParams& p, int tm) {
 }
 
 
+// Eight consecutive output columns of one row: bias, activation / gate + residual / accumulation, store.  `v` holds the
+// scaled accumulator values, `c_row` is where the row's output starts (column 0), `gate_row` its gate row.
+__device__ __forceinline__ void epilogue_vec(const GemmParams& p, float (&v)[8], int row, int col, bf16* c_row,
+                                             const float* gate_row) {
+  if (p.bias) {
+    uint4 bv = *reinterpret_cast<const uint4*>(p.bias + col);
+    const uint32_t* bu = reinterpret_cast<const uint32_t*>(&bv);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      float2 f = unpack_bf16(bu[j]);
+      v[2 * j] += f.x;
+      v[2 * j + 1] += f.y;
+    }
+  }
+  if (p.epi == EPI_GELU || p.epi == EPI_SILU) {
+    if (p.aux_out) {
+      uint4 o;
+      o.x = pack_bf16(v[0], v[1]);
+      o.y = pack_bf16(v[2], v[3]);
+      o.z = pack_bf16(v[4], v[5]);
+      o.w = pack_bf16(v[6], v[7]);
+      *reinterpret_cast<uint4*>(p.aux_out + (long long)row * p.ldc + col) = o;
+    }
+    if (p.epi == EPI_GELU) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = gelu_tanh(v[j]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = silu(v[j]);
+    }
+  } else if (p.epi == EPI_GATE_RES) {
+    if (p.aux_out) {  // keep the un-gated branch output: its gradient needs it
+      uint4 o;
+      o.x = pack_bf16(v[0], v[1]);
+      o.y = pack_bf16(v[2], v[3]);
+      o.z = pack_bf16(v[4], v[5]);
+      o.w = pack_bf16(v[6], v[7]);
+      *reinterpret_cast<uint4*>(p.aux_out + (long long)row * p.ldc + col) = o;
+    }
+    uint4 rv = *reinterpret_cast<const uint4*>(p.residual + (long long)row * p.ldr + col);
+    const uint32_t* ru = reinterpret_cast<const uint32_t*>(&rv);
+    float4 g0 = *reinterpret_cast<const float4*>(gate_row + col);
+    float4 g1 = *reinterpret_cast<const float4*>(gate_row + col + 4);
+    const float gg[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      float2 f = unpack_bf16(ru[j]);
+      v[2 * j] = f.x + gg[2 * j] * v[2 * j];
+      v[2 * j + 1] = f.y + gg[2 * j + 1] * v[2 * j + 1];
+    }
+  } else if (p.epi == EPI_ACCUM) {
+    if (p.c_fp32) {
+      const float* cp = reinterpret_cast<const float*>(p.C) + (long long)row * p.ldc + col;
+      float4 c0 = *reinterpret_cast<const float4*>(cp);
+      float4 c1 = *reinterpret_cast<const float4*>(cp + 4);
+      v[0] += c0.x; v[1] += c0.y; v[2] += c0.z; v[3] += c0.w;
+      v[4] += c1.x; v[5] += c1.y; v[6] += c1.z; v[7] += c1.w;
+    } else {
+      uint4 cv = *reinterpret_cast<const uint4*>(reinterpret_cast<const bf16*>(p.C) +
+                                                 (long long)row * p.ldc + col);
+      const uint32_t* cu = reinterpret_cast<const uint32_t*>(&cv);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        float2 f = unpack_bf16(cu[j]);
+        v[2 * j] += f.x;
+        v[2 * j + 1] += f.y;
+      }
+    }
+  }
+  if (p.c_fp32) {
+    float* cp = reinterpret_cast<float*>(p.C) + (long long)row * p.ldc + col;
+    *reinterpret_cast<float4*>(cp) = make_float4(v[0], v[1], v[2], v[3]);
+    *reinterpret_cast<float4*>(cp + 4) = make_float4(v[4], v[5], v[6], v[7]);
+  } else {
+    uint4 o;
+    o.x = pack_bf16(v[0], v[1]);
+    o.y = pack_bf16(v[2], v[3]);
+    o.z = pack_bf16(v[4], v[5]);
+    o.w = pack_bf16(v[6], v[7]);
+    *reinterpret_cast<uint4*>(c_row + col) = o;
+  }
+}
+
 // Epilogue of one 128-row accumulator tile for the warp that owns lane quarter `q` and column group `eg` (of 2):
 // `acc` is the tensor-memory address of the tile's first column for this quarter, `row` the global output row of
 // this lane, `c_row` where that row's output starts (column 0), `n0` the tile's first output column.
@@ -92,83 +175,7 @@ __device__ __forceinline__ void epilogue_tile(const GemmParams& p, uint32_t acc,
       float v[8];
 #pragma unroll
       for (int j = 0; j < 8; ++j) v[j] = __uint_as_float(r[g * 8 + j]) * p.alpha;
-      if (p.bias) {
-        uint4 bv = *reinterpret_cast<const uint4*>(p.bias + col);
-        const uint32_t* bu = reinterpret_cast<const uint32_t*>(&bv);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          float2 f = unpack_bf16(bu[j]);
-          v[2 * j] += f.x;
-          v[2 * j + 1] += f.y;
-        }
-      }
-      if (p.epi == EPI_GELU || p.epi == EPI_SILU) {
-        if (p.aux_out) {
-          uint4 o;
-          o.x = pack_bf16(v[0], v[1]);
-          o.y = pack_bf16(v[2], v[3]);
-          o.z = pack_bf16(v[4], v[5]);
-          o.w = pack_bf16(v[6], v[7]);
-          *reinterpret_cast<uint4*>(p.aux_out + (long long)row * p.ldc + col) = o;
-        }
-        if (p.epi == EPI_GELU) {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) v[j] = gelu_tanh(v[j]);
-        } else {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) v[j] = silu(v[j]);
-        }
-      } else if (p.epi == EPI_GATE_RES) {
-        if (p.aux_out) {  // keep the un-gated branch output: its gradient needs it
-          uint4 o;
-          o.x = pack_bf16(v[0], v[1]);
-          o.y = pack_bf16(v[2], v[3]);
-          o.z = pack_bf16(v[4], v[5]);
-          o.w = pack_bf16(v[6], v[7]);
-          *reinterpret_cast<uint4*>(p.aux_out + (long long)row * p.ldc + col) = o;
-        }
-        uint4 rv = *reinterpret_cast<const uint4*>(p.residual + (long long)row * p.ldr + col);
-        const uint32_t* ru = reinterpret_cast<const uint32_t*>(&rv);
-        float4 g0 = *reinterpret_cast<const float4*>(gate_row + col);
-        float4 g1 = *reinterpret_cast<const float4*>(gate_row + col + 4);
-        const float gg[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          float2 f = unpack_bf16(ru[j]);
-          v[2 * j] = f.x + gg[2 * j] * v[2 * j];
-          v[2 * j + 1] = f.y + gg[2 * j + 1] * v[2 * j + 1];
-        }
-      } else if (p.epi == EPI_ACCUM) {
-        if (p.c_fp32) {
-          const float* cp = reinterpret_cast<const float*>(p.C) + (long long)row * p.ldc + col;
-          float4 c0 = *reinterpret_cast<const float4*>(cp);
-          float4 c1 = *reinterpret_cast<const float4*>(cp + 4);
-          v[0] += c0.x; v[1] += c0.y; v[2] += c0.z; v[3] += c0.w;
-          v[4] += c1.x; v[5] += c1.y; v[6] += c1.z; v[7] += c1.w;
-        } else {
-          uint4 cv = *reinterpret_cast<const uint4*>(reinterpret_cast<const bf16*>(p.C) +
-                                                     (long long)row * p.ldc + col);
-          const uint32_t* cu = reinterpret_cast<const uint32_t*>(&cv);
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            float2 f = unpack_bf16(cu[j]);
-            v[2 * j] += f.x;
-            v[2 * j + 1] += f.y;
-          }
-        }
-      }
-      if (p.c_fp32) {
-        float* cp = reinterpret_cast<float*>(p.C) + (long long)row * p.ldc + col;
-        *reinterpret_cast<float4*>(cp) = make_float4(v[0], v[1], v[2], v[3]);
-        *reinterpret_cast<float4*>(cp + 4) = make_float4(v[4], v[5], v[6], v[7]);
-      } else {
-        uint4 o;
-        o.x = pack_bf16(v[0], v[1]);
-        o.y = pack_bf16(v[2], v[3]);
-        o.z = pack_bf16(v[4], v[5]);
-        o.w = pack_bf16(v[6], v[7]);
-        *reinterpret_cast<uint4*>(c_row + col) = o;
-      }
+      epilogue_vec(p, v, row, col, c_row, gate_row);
     }
     __syncwarp();  // tcgen05.ld is warp-collective: reconverge before the next chunk
   }
@@ -237,4 +244,19 @@ __device__ __forceinline__ void epilogue_tile_qkv(const GemmParams& p, uint32_t 
   }
 }
 
+// Products whose 128 x 128 output tiles would leave half of the SMs idle are cut along K (csrc/gemm_splitk.cu): by how
+// much, or 1.  Each part keeps at least four 64-wide steps, below that the start-up of a CTA outweighs its loop.
+inline int splitk_factor(int M, int N, int K, int sms) {
+  const long long tiles = (long long)((M + 127) / 128) * ((N + 127) / 128);
+  const int num_kb = (K + BK - 1) / BK;
+  int s = 1;
+  while (s < 8 && tiles * s * 2 <= sms && num_kb >= 8 * s) s *= 2;
+  return s;
+}
+
 }  // namespace tt_gemm
+
+// same contract as tt_gemm_bf16, with the K range cut into `split` parts; tensor maps with boxes of 64 x 128 (K-major) or
+// 64 x 64 (MN-major) elements
+int tt_gemm_splitk(const CUtensorMap& tmA, const CUtensorMap& tmB, int a_mn, int b_mn, const tt_gemm::GemmParams& p, int split,
+                   cudaStream_t stream);
