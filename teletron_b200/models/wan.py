@@ -28,6 +28,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from .. import ops
+from ..ops.gemm import pair_gemm
 from ..parallel import recompute as rc
 from ..parallel.ulysses import UlyssesContext
 
@@ -267,6 +268,9 @@ class DiTBlock(nn.Module):
 
     def forward(self, x2d, context, t_mod, freqs, batch: int, cp: Optional[UlyssesContext]):
         rows_per_batch = x2d.shape[0] // batch
+        out = wan_block_infer(self, x2d, context, t_mod, freqs, batch, cp)
+        if out is not None:
+            return out
         e = self.modulation.float() + t_mod  # [B, 6, C] fp32
         # each norm also hands back its input for the residual branch, so that the residual's gradient is added
         # inside the norm's backward kernel
@@ -277,6 +281,61 @@ class DiTBlock(nn.Module):
         h, xr = ops.adaln_res(x2d, e[:, 4], e[:, 3], rows_per_batch, self.eps)
         return ops.ffn(h, self.ffn[0].weight, self.ffn[0].bias, self.ffn[2].weight, self.ffn[2].bias, xr, e[:, 5],
                        rows_per_batch, act="gelu")
+
+
+def _block_params(blk: DiTBlock):
+    """The block's parameters in the order of csrc/wan_block.cu."""
+    sa, ca, f1, f2 = blk.self_attn, blk.cross_attn, blk.ffn[0], blk.ffn[2]
+    return (blk.modulation, sa.qkv.weight, sa.qkv.bias, sa.norm_q.weight, sa.norm_k.weight, sa.o.weight, sa.o.bias,
+            blk.norm3.weight, blk.norm3.bias, ca.q.weight, ca.q.bias, ca.kv.weight, ca.kv.bias, ca.norm_q.weight,
+            ca.norm_k.weight, ca.o.weight, ca.o.bias, f1.weight, f1.bias, f2.weight, f2.bias)
+
+
+def wan_block_infer(blk: DiTBlock, x2d, context, t_mod, freqs, batch: int, cp):
+    """The block without gradients as one native call (csrc/wan_block.cu), or None where the op layer has to run:
+    with gradients, on CPU, under context parallelism or tracing, with image tokens, with hooks on inner modules, or
+    for tensors and parameters that are not dense bf16 of one device."""
+    if torch.is_grad_enabled() or not x2d.is_cuda or cp is not None or blk.self_attn.head_dim != 128:
+        return None
+    if blk.cross_attn.has_image_input or context.dim() != 3 or torch.is_autocast_enabled("cuda"):
+        return None
+    if torch.jit.is_tracing() or torch.compiler.is_compiling() or torch.nn.modules.module._has_any_global_hook():
+        return None
+    if any(type(t) is not torch.Tensor or torch._C._functorch.is_functorch_wrapped_tensor(t)
+           for t in (x2d, context, t_mod, freqs)):
+        return None
+    if torch.autograd.forward_ad._current_level >= 0:
+        return None
+    bf16 = torch.bfloat16
+    C, dev, (B, Lc, Cc) = blk.dim, x2d.device, context.shape
+    if x2d.dtype != bf16 or x2d.dim() != 2 or x2d.stride(1) != 1 or x2d.stride(0) % 8 or x2d.shape[0] % batch:
+        return None
+    if context.dtype != bf16 or not context.is_contiguous() or (B, Cc) != (batch, C) or context.device != dev:
+        return None
+    if t_mod.dtype != torch.float32 or not t_mod.is_contiguous() or t_mod.shape != (batch, 6, C) or t_mod.device != dev:
+        return None
+    if freqs.dtype != torch.float32 or not freqs.is_contiguous() or freqs.shape[1:] != (64, 2) or freqs.device != dev:
+        return None
+    params = _block_params(blk)
+    for p in params:
+        if p is None or p.dtype != bf16 or p.device != dev or not p.is_contiguous():
+            return None
+    if any(m._forward_hooks or m._forward_pre_hooks for m in blk.modules() if m is not blk):
+        return None
+    lib, S, F_ = ops._lib, x2d.shape[0] // batch, blk.ffn[0].weight.shape[0]
+    ptrs = [p.data_ptr() for p in params]
+    if any(a & 15 for a in ptrs) or (x2d.data_ptr() | context.data_ptr() | freqs.data_ptr()) & 15 or F_ % 8 or S == 0:
+        return None
+    L = lib.lib()
+    dims = (lib.c_int(batch), lib.c_int(S), lib.c_int(Lc), lib.c_int(C), lib.c_int(blk.self_attn.num_heads), lib.c_int(F_))
+    L.tt_wan_block_workspace.restype = lib.c_ll
+    work = torch.empty(L.tt_wan_block_workspace(*dims), dtype=torch.uint8, device=dev)
+    out = torch.empty((x2d.shape[0], C), dtype=bf16, device=dev)
+    lib.check(L.tt_wan_block_fwd(
+        lib.ptr(x2d), lib.c_ll(x2d.stride(0)), lib.ptr(out), lib.ptr(context), lib.ptr(t_mod), lib.ptr(freqs),
+        lib.c_int(freqs.shape[0]), (lib.c_ll * len(ptrs))(*ptrs), *dims, lib.c_float(blk.eps), lib.c_int(int(pair_gemm())),
+        lib.ptr(work), lib.ptr(lib.status_word(dev)), lib.stream()), "tt_wan_block_fwd")
+    return out
 
 
 class ImageEmbedMLP(nn.Module):

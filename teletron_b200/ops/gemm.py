@@ -27,6 +27,10 @@ def set_pair_gemm(on: bool) -> bool:
     return old
 
 
+def pair_gemm() -> bool:
+    return _PAIR
+
+
 def _logical(a: torch.Tensor, mn_major: bool) -> torch.Tensor:
     return a.t() if mn_major else a
 
