@@ -34,21 +34,6 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
   for (int i = 0; i < NT / 32; ++i) t += red[i];
   return t;
 }
-__device__ __forceinline__ float2 block_sum2(float2 v, float2* red) {
-  v.x = warp_sum(v.x);
-  v.y = warp_sum(v.y);
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  __syncthreads();
-  if (l == 0) red[w] = v;
-  __syncthreads();
-  float2 t = make_float2(0.f, 0.f);
-#pragma unroll
-  for (int i = 0; i < NT / 32; ++i) {
-    t.x += red[i].x;
-    t.y += red[i].y;
-  }
-  return t;
-}
 
 __device__ __forceinline__ void load8(const bf16* p, float (&v)[8]) {
   uint4 u = *reinterpret_cast<const uint4*>(p);
@@ -74,6 +59,21 @@ __device__ __forceinline__ void loadf8(const float* p, float (&v)[8]) {
   v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
   v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
 }
+
+__device__ __forceinline__ uint4 ldraw(const bf16* p) { return *reinterpret_cast<const uint4*>(p); }
+__device__ __forceinline__ void unpack8(const uint4& u, float (&v)[8]) {
+  const uint32_t* w = reinterpret_cast<const uint32_t*>(&u);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float2 f = unpack_bf16(w[j]);
+    v[2 * j] = f.x;
+    v[2 * j + 1] = f.y;
+  }
+}
+
+// makes the compiler forget what it knows about a packed vector: the next pass unpacks it again instead of keeping the
+// floats of the last one alive (or spilled)
+__device__ __forceinline__ void forget(uint4& u) { asm volatile("" : "+r"(u.x), "+r"(u.y), "+r"(u.z), "+r"(u.w)); }
 
 // ------------------------------------------------------------------ AdaLN forward
 template <int VPT>
@@ -229,14 +229,17 @@ adaln_fwd_warp_kernel(const bf16* __restrict__ x, long long ldx, bf16* __restric
 
 // ------------------------------------------------------------------ AdaLN backward
 // grid = (chunks, batch). CTA (chunk, b) owns rows [b*rpb + chunk*rpc, min(.. + rpc, (b+1)*rpb)).
-template <int VPT>
-__global__ void __launch_bounds__(NT)
+// A CTA walks its rows one after the other, so what bounds it is the latency of a row: the next row's loads are issued
+// before this row's reduction, the reduction buffer alternates (one barrier per row), and rows stay packed (the values
+// are unpacked again for the second pass) so that two or more CTAs fit an SM.
+template <int VPT, int NTH, int MINB>
+__global__ void __launch_bounds__(NTH, MINB)
 adaln_bwd_kernel(const bf16* __restrict__ dy, long long lddy, const bf16* __restrict__ x,
                  long long ldx, const float* __restrict__ mean_in, const float* __restrict__ rstd_in,
                  const float* __restrict__ mul, long long mod_ld, int plus_one, bf16* __restrict__ dx,
                  long long lddx, const bf16* __restrict__ dx_add, long long ldadd,
                  float* __restrict__ partial, int C, int rows_per_batch, int rows_per_chunk) {
-  __shared__ float2 red[NT / 32];
+  __shared__ float2 red[2][NTH / 32];
   const int nvec = C >> 3;
   const float invC = 1.f / (float)C;
   const int b = blockIdx.y;
@@ -244,9 +247,27 @@ adaln_bwd_kernel(const bf16* __restrict__ dy, long long lddy, const bf16* __rest
   const int r0 = chunk * rows_per_chunk;
   const int r1 = min(r0 + rows_per_chunk, rows_per_batch);
   float m[VPT][8], acc_mul[VPT][8], acc_add[VPT][8];
+  uint4 nd[VPT], nx[VPT];
+  float nmean = 0.f, nrstd = 0.f;
+  auto fetch = [&](int r) {
+    const long long row = (long long)b * rows_per_batch + r;
+#pragma unroll
+    for (int k = 0; k < VPT; ++k) {
+      const int vec = threadIdx.x + k * NTH;
+      nd[k] = make_uint4(0, 0, 0, 0);
+      nx[k] = make_uint4(0, 0, 0, 0);
+      if (vec < nvec) {
+        nd[k] = ldraw(dy + row * lddy + vec * 8);
+        nx[k] = ldraw(x + row * ldx + vec * 8);
+      }
+    }
+    nmean = mean_in[row];
+    nrstd = rstd_in[row];
+  };
+  if (r0 < r1) fetch(r0);
 #pragma unroll
   for (int k = 0; k < VPT; ++k) {
-    const int vec = threadIdx.x + k * NT;
+    const int vec = threadIdx.x + k * NTH;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       acc_mul[k][j] = 0.f;
@@ -261,42 +282,58 @@ adaln_bwd_kernel(const bf16* __restrict__ dy, long long lddy, const bf16* __rest
   }
   for (int r = r0; r < r1; ++r) {
     const long long row = (long long)b * rows_per_batch + r;
-    const float mean = mean_in[row], rstd = rstd_in[row];
-    float g[VPT][8], xh[VPT][8];
+    uint4 cd[VPT], cx[VPT], ce[VPT];
+    const float mean = nmean, rstd = nrstd;
+#pragma unroll
+    for (int k = 0; k < VPT; ++k) {
+      cd[k] = nd[k];
+      cx[k] = nx[k];
+      const int vec = threadIdx.x + k * NTH;
+      ce[k] = make_uint4(0, 0, 0, 0);
+      if (dx_add && vec < nvec) ce[k] = ldraw(dx_add + row * ldadd + vec * 8);
+    }
+    if (r + 1 < r1) fetch(r + 1);
     float2 s = make_float2(0.f, 0.f);
 #pragma unroll
     for (int k = 0; k < VPT; ++k) {
-      const int vec = threadIdx.x + k * NT;
-      if (vec < nvec) {
+      if (threadIdx.x + k * NTH < nvec) {
         float d[8], xv[8];
-        load8(dy + row * lddy + vec * 8, d);
-        load8(x + row * ldx + vec * 8, xv);
+        unpack8(cd[k], d);
+        unpack8(cx[k], xv);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-          xh[k][j] = (xv[j] - mean) * rstd;
-          acc_mul[k][j] += d[j] * xh[k][j];
+          const float xh = (xv[j] - mean) * rstd, g = d[j] * m[k][j];
+          acc_mul[k][j] += d[j] * xh;
           acc_add[k][j] += d[j];
-          g[k][j] = d[j] * m[k][j];
-          s.x += g[k][j];
-          s.y += g[k][j] * xh[k][j];
+          s.x += g;
+          s.y += g * xh;
         }
       }
     }
-    s = block_sum2(s, red);
-    const float c1 = s.x * invC, c2 = s.y * invC;
+    s.x = warp_sum(s.x);
+    s.y = warp_sum(s.y);
+    float2* rd = red[r & 1];
+    if ((threadIdx.x & 31) == 0) rd[threadIdx.x >> 5] = s;
+    __syncthreads();
+    float2 t = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < NTH / 32; ++i) {
+      t.x += rd[i].x;
+      t.y += rd[i].y;
+    }
+    const float c1 = t.x * invC, c2 = t.y * invC;
 #pragma unroll
     for (int k = 0; k < VPT; ++k) {
-      const int vec = threadIdx.x + k * NT;
+      const int vec = threadIdx.x + k * NTH;
       if (vec < nvec) {
-        float o[8];
+        float d[8], xv[8], e[8], o[8];
+        forget(cd[k]);
+        forget(cx[k]);
+        unpack8(cd[k], d);
+        unpack8(cx[k], xv);
+        unpack8(ce[k], e);  // the residual-branch gradient, zero without one
 #pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] = rstd * (g[k][j] - c1 - xh[k][j] * c2);
-        if (dx_add) {  // fold the residual-branch gradient into the same pass
-          float e[8];
-          load8(dx_add + row * ldadd + vec * 8, e);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) o[j] += e[j];
-        }
+        for (int j = 0; j < 8; ++j) o[j] = rstd * (d[j] * m[k][j] - c1 - (xv[j] - mean) * rstd * c2) + e[j];
         store8(dx + row * lddx + vec * 8, o);
       }
     }
@@ -306,7 +343,7 @@ adaln_bwd_kernel(const bf16* __restrict__ dy, long long lddy, const bf16* __rest
     float* pa = pm + C;
 #pragma unroll
     for (int k = 0; k < VPT; ++k) {
-      const int vec = threadIdx.x + k * NT;
+      const int vec = threadIdx.x + k * NTH;
       if (vec < nvec) {
         *reinterpret_cast<float4*>(pm + vec * 8) = make_float4(acc_mul[k][0], acc_mul[k][1], acc_mul[k][2], acc_mul[k][3]);
         *reinterpret_cast<float4*>(pm + vec * 8 + 4) = make_float4(acc_mul[k][4], acc_mul[k][5], acc_mul[k][6], acc_mul[k][7]);
@@ -353,26 +390,23 @@ colsum_partials_kernel(const float* __restrict__ partial, float* __restrict__ ou
 // ------------------------------------------------------------------ RMSNorm + RoPE
 // norm_dim == C : statistics over the whole row; norm_dim == D : per head (16 threads own
 // one head of 128). w may be null (no norm), freqs may be null (no rotary).
-template <int VPT, bool BWD>
+template <int VPT>
 __global__ void __launch_bounds__(NT)
-rmsrope_kernel(const bf16* __restrict__ in, long long ldi, const bf16* __restrict__ xsave,
-               long long ldx, bf16* __restrict__ out, long long ldo, const float* __restrict__ w,
+rmsrope_kernel(const bf16* __restrict__ in, long long ldi, bf16* __restrict__ out, long long ldo, const float* __restrict__ w,
                const float2* __restrict__ freqs, int freq_rows, float* __restrict__ rstd_io,
-               float* __restrict__ partial, int rows, int C, int D, int per_head, float eps,
+               int rows, int C, int D, int per_head, float eps,
                int rows_per_cta, const TTScatter sc, const float* __restrict__ ssq = nullptr, int ssq_n = 0,
                long long ssq_ld = 0) {
   __shared__ float red[NT / 32];
   const int nvec = C >> 3;
   const int vec_per_head = D >> 3;
   const int H = C / D;
-  float accw[VPT][8];
   float wv[VPT][8];
 #pragma unroll
   for (int k = 0; k < VPT; ++k) {
     const int vec = threadIdx.x + k * NT;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      accw[k][j] = 0.f;
       wv[k][j] = 1.f;
     }
     if (w && vec < nvec) loadf8(w + (per_head ? (vec % vec_per_head) * 8 : vec * 8), wv[k]);
@@ -380,7 +414,7 @@ rmsrope_kernel(const bf16* __restrict__ in, long long ldi, const bf16* __restric
   const int r0 = blockIdx.x * rows_per_cta;
   const int r1 = min(r0 + rows_per_cta, rows);
   for (int row = r0; row < r1; ++row) {
-    float v[VPT][8];  // forward: x ; backward: dy then g
+    float v[VPT][8];
     float cs[VPT][8];
     const float2* frow = freqs ? freqs + (long long)(row % freq_rows) * (D >> 1) : nullptr;
 #pragma unroll
@@ -391,7 +425,7 @@ rmsrope_kernel(const bf16* __restrict__ in, long long ldi, const bf16* __restric
         if (frow) loadf8(reinterpret_cast<const float*>(frow + (vec % vec_per_head) * 4), cs[k]);
       }
     }
-    if (!BWD) {
+    {
       float rs[VPT];
       if (w) {
         float ss[VPT];
@@ -456,80 +490,6 @@ rmsrope_kernel(const bf16* __restrict__ in, long long ldi, const bf16* __restric
             store8(scatter_dst(sc, row / sc.S_l, row % sc.S_l, hd) + (col - hd * D), o);
           }
         }
-      }
-    } else {
-      // backward: v = dy. un-rotate, then norm backward from saved x and rstd.
-      float xh[VPT][8];
-      float dot[VPT];
-      float tot = 0.f;
-#pragma unroll
-      for (int k = 0; k < VPT; ++k) {
-        dot[k] = 0.f;
-        const int vec = threadIdx.x + k * NT;
-        if (vec < nvec) {
-          if (frow) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const float c = cs[k][2 * j], s = cs[k][2 * j + 1];
-              const float a = v[k][2 * j], b = v[k][2 * j + 1];
-              v[k][2 * j] = a * c + b * s;
-              v[k][2 * j + 1] = -a * s + b * c;
-            }
-          }
-          if (w) {
-            float xv[8];
-            load8(xsave + (long long)row * ldx + vec * 8, xv);
-            const float r = per_head ? rstd_io[(long long)row * H + vec / vec_per_head] : rstd_io[row];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              xh[k][j] = xv[j] * r;
-              accw[k][j] += v[k][j] * xh[k][j];
-              v[k][j] *= wv[k][j];
-              dot[k] += v[k][j] * xh[k][j];
-            }
-          }
-        }
-        tot += dot[k];
-      }
-      if (w) {
-        float full = 0.f;
-        if (!per_head) full = block_sum(tot, red) / (float)C;
-#pragma unroll
-        for (int k = 0; k < VPT; ++k) {
-          const int vec = threadIdx.x + k * NT;
-          float sdot;
-          if (per_head) {
-            float t = dot[k];
-            for (int o = vec_per_head >> 1; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-            sdot = t / (float)D;
-          } else {
-            sdot = full;
-          }
-          if (vec < nvec) {
-            const float r = per_head ? rstd_io[(long long)row * H + vec / vec_per_head] : rstd_io[row];
-            float o[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) o[j] = r * (v[k][j] - xh[k][j] * sdot);
-            store8(out + (long long)row * ldo + vec * 8, o);
-          }
-        }
-      } else {
-#pragma unroll
-        for (int k = 0; k < VPT; ++k) {
-          const int vec = threadIdx.x + k * NT;
-          if (vec < nvec) store8(out + (long long)row * ldo + vec * 8, v[k]);
-        }
-      }
-    }
-  }
-  if (BWD && partial && w) {
-    float* pw = partial + (long long)blockIdx.x * C;
-#pragma unroll
-    for (int k = 0; k < VPT; ++k) {
-      const int vec = threadIdx.x + k * NT;
-      if (vec < nvec) {
-        *reinterpret_cast<float4*>(pw + vec * 8) = make_float4(accw[k][0], accw[k][1], accw[k][2], accw[k][3]);
-        *reinterpret_cast<float4*>(pw + vec * 8 + 4) = make_float4(accw[k][4], accw[k][5], accw[k][6], accw[k][7]);
       }
     }
   }
@@ -604,9 +564,17 @@ TT_API int tt_adaln_bwd(const void* dy, long long lddy, const void* x, long long
            "adaln_bwd: misaligned pointer");
   const int rpc = (rows_per_batch + chunks - 1) / chunks;
   dim3 grid(chunks, batch);
-  TT_DISPATCH_VPT(vpt_for(C), adaln_bwd_kernel<VPT><<<grid, NT, 0, stream>>>(
-      (const bf16*)dy, lddy, (const bf16*)x, ldx, mean, rstd, mul, mod_ld, plus_one, (bf16*)dx, lddx,
-      (const bf16*)dx_add, ldadd, partial, C, rows_per_batch, rpc));
+#define TT_ADALN_BWD(V, T, B)                                                                                           \
+  adaln_bwd_kernel<V, T, B><<<grid, T, 0, stream>>>((const bf16*)dy, lddy, (const bf16*)x, ldx, mean, rstd, mul, mod_ld, \
+                                                    plus_one, (bf16*)dx, lddx, (const bf16*)dx_add, ldadd, partial, C,   \
+                                                    rows_per_batch, rpc)
+  // few idle lanes at the usual widths (1536, 2048, 3072, 5120) and at most two vectors per thread
+  if (C <= 1536) TT_ADALN_BWD(1, 192, 5);
+  else if (C <= 2048) TT_ADALN_BWD(1, 256, 4);
+  else if (C <= 3072) TT_ADALN_BWD(1, 384, 2);
+  else if (C <= 5120) TT_ADALN_BWD(2, 320, 2);
+  else TT_ADALN_BWD(2, 384, 1);
+#undef TT_ADALN_BWD
   TT_LAUNCH_CHECK();
   if (partial && (dmul || dadd)) {
     dim3 g2((C + 31) / 32, batch);
@@ -633,10 +601,12 @@ TT_API int tt_colsum_partials(const float* partial, float* out, int groups, int 
 }
 
 // ------------------------------------------------------------------ RMSNorm + RoPE, one row per warp
-// Full-row statistics only (Wan q / k norm), C = NV * 256: each lane holds NV 16-byte vectors of the row, the
-// reductions are warp shuffles, eight rows per CTA are in flight.  The row-per-CTA kernel above reached a third of the
-// copy bandwidth at C = 1536 (two block barriers per 3 KB row).  The weight row lives in shared memory.
-template <int NV>
+// C = NV * 256: each lane holds NV 16-byte vectors of the row (packed: the 10 KB of a 5120-wide row are 80
+// registers per lane), the reductions are
+// warp shuffles (over the 8 or 16 lanes of a head with PER_HEAD), eight rows per CTA are in flight.  The row-per-CTA
+// kernel above reached a third of the copy bandwidth at C = 1536 (two block barriers per 3 KB row), half of it at 3072
+// and 5120.  The weight row lives in shared memory.
+template <int NV, bool PER_HEAD>
 __global__ void __launch_bounds__(NT, 2)
 rmsrope_fwd_warp_kernel(const bf16* __restrict__ in, long long ldi, bf16* __restrict__ out, long long ldo,
                         const float* __restrict__ w, const float2* __restrict__ freqs, int freq_rows,
@@ -646,25 +616,28 @@ rmsrope_fwd_warp_kernel(const bf16* __restrict__ in, long long ldi, bf16* __rest
   __shared__ __align__(16) float w_s[C];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int vec_per_head = D >> 3;
-  for (int i = threadIdx.x; i < C; i += NT) w_s[i] = w ? w[i] : 1.f;
+  for (int i = threadIdx.x; i < C; i += NT) w_s[i] = w ? w[PER_HEAD ? i % D : i] : 1.f;
   __syncthreads();
   for (int row = blockIdx.x * (NT / 32) + warp; row < rows; row += gridDim.x * (NT / 32)) {
-    float v[NV][8];
+    uint4 raw[NV];
     const float2* frow = freqs ? freqs + (long long)(row % freq_rows) * (D >> 1) : nullptr;
     const bf16* xr = in + (long long)row * ldi;
 #pragma unroll
-    for (int k = 0; k < NV; ++k) load8(xr + (lane + k * 32) * 8, v[k]);
+    for (int k = 0; k < NV; ++k) raw[k] = ldraw(xr + (lane + k * 32) * 8);
     float r = 1.f;
-    if (w) {
+    if (!PER_HEAD && w) {
       float tot = 0.f;
       if (ssq) {  // row statistics already produced (per 128-column piece) by the GEMM that wrote this row
         for (int j = 0; j < ssq_n; ++j) tot += ssq[(long long)row * ssq_ld + j];
       } else {
         float ss = 0.f;
 #pragma unroll
-        for (int k = 0; k < NV; ++k)
+        for (int k = 0; k < NV; ++k) {
+          float v[8];
+          unpack8(raw[k], v);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) ss += v[k][j] * v[k][j];
+          for (int j = 0; j < 8; ++j) ss += v[j] * v[j];
+        }
         tot = warp_sum(ss);
       }
       r = rsqrtf(tot / (float)C + eps);
@@ -673,10 +646,20 @@ rmsrope_fwd_warp_kernel(const bf16* __restrict__ in, long long ldi, bf16* __rest
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
       const int vec = lane + k * 32;
-      float o[8], wk[8];
+      float v[8], o[8], wk[8];
+      forget(raw[k]);
+      unpack8(raw[k], v);
+      if (PER_HEAD && w) {
+        float t = 0.f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) t += v[j] * v[j];
+        for (int q = vec_per_head >> 1; q > 0; q >>= 1) t += __shfl_xor_sync(0xffffffffu, t, q);
+        r = rsqrtf(t / (float)D + eps);
+        if ((lane & (vec_per_head - 1)) == 0 && rstd_io) rstd_io[(long long)row * (C / D) + vec / vec_per_head] = r;
+      }
       loadf8(&w_s[vec * 8], wk);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) o[j] = v[k][j] * r * wk[j];
+      for (int j = 0; j < 8; ++j) o[j] = v[j] * r * wk[j];
       if (frow) {
         float cs[8];
         loadf8(reinterpret_cast<const float*>(frow + (vec % vec_per_head) * 4), cs);
@@ -783,6 +766,134 @@ rmsrope_bwd_warp_kernel(const bf16* __restrict__ dy, long long lddy, const bf16*
   }
 }
 
+// Backward with one row per CTA step, for what the warp kernel does not take (wide rows, per-head statistics, or no norm
+// at all: w == null, only the rotation is undone): the next row's loads are issued
+// before this row's reduction and the reduction buffer alternates, see adaln_bwd_kernel.  Thread t holds vectors t and
+// t + NTH of every row, and with them their weight-gradient sums.
+template <int VPT, int NTH, int MINB>
+__global__ void __launch_bounds__(NTH, MINB)
+rmsrope_bwd_row_kernel(const bf16* __restrict__ dy, long long lddy, const bf16* __restrict__ xsave, long long ldx,
+                       bf16* __restrict__ dx, long long lddx, const float* __restrict__ w,
+                       const float2* __restrict__ freqs, int freq_rows, const float* __restrict__ rstd_in,
+                       float* __restrict__ partial, int rows, int C, int D, int per_head, int rows_per_cta) {
+  __shared__ float red[2][NTH / 32];
+  const int nvec = C >> 3, vph = D >> 3, H = C / D;
+  float wv[VPT][8], acc[VPT][8];
+#pragma unroll
+  for (int k = 0; k < VPT; ++k) {
+    const int vec = threadIdx.x + k * NTH;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[k][j] = wv[k][j] = 0.f;
+    if (w && vec < nvec) loadf8(w + (per_head ? (vec % vph) * 8 : vec * 8), wv[k]);
+  }
+  const int r0 = blockIdx.x * rows_per_cta, r1 = min(r0 + rows_per_cta, rows);
+  uint4 nd[VPT], nx[VPT];
+  float nr[VPT];
+  auto fetch = [&](int row) {
+#pragma unroll
+    for (int k = 0; k < VPT; ++k) {
+      const int vec = threadIdx.x + k * NTH;
+      nd[k] = make_uint4(0, 0, 0, 0);
+      nx[k] = make_uint4(0, 0, 0, 0);
+      nr[k] = 0.f;
+      if (vec < nvec) {
+        nd[k] = ldraw(dy + (long long)row * lddy + vec * 8);
+        if (w) {
+          nx[k] = ldraw(xsave + (long long)row * ldx + vec * 8);
+          nr[k] = rstd_in[per_head ? (long long)row * H + vec / vph : row];
+        }
+      }
+    }
+  };
+  if (r0 < r1) fetch(r0);
+  for (int row = r0; row < r1; ++row) {
+    uint4 cx[VPT];
+    float g[VPT][8], rs[VPT], dot[VPT];
+    const float2* frow = freqs ? freqs + (long long)(row % freq_rows) * (D >> 1) : nullptr;
+    float tot = 0.f;
+#pragma unroll
+    for (int k = 0; k < VPT; ++k) {
+      const int vec = threadIdx.x + k * NTH;
+      unpack8(nd[k], g[k]);
+      cx[k] = nx[k];
+      rs[k] = nr[k];
+      if (frow && vec < nvec) {
+        float cs[8];
+        loadf8(reinterpret_cast<const float*>(frow + (vec % vph) * 4), cs);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float c = cs[2 * j], sn = cs[2 * j + 1], a = g[k][2 * j], b = g[k][2 * j + 1];
+          g[k][2 * j] = a * c + b * sn;
+          g[k][2 * j + 1] = -a * sn + b * c;
+        }
+      }
+    }
+    if (row + 1 < r1) fetch(row + 1);
+    if (!w) {
+#pragma unroll
+      for (int k = 0; k < VPT; ++k) {
+        const int vec = threadIdx.x + k * NTH;
+        if (vec < nvec) store8(dx + (long long)row * lddx + vec * 8, g[k]);
+      }
+      continue;
+    }
+#pragma unroll
+    for (int k = 0; k < VPT; ++k) {
+      float xv[8];
+      unpack8(cx[k], xv);
+      dot[k] = 0.f;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float xh = xv[j] * rs[k];
+        acc[k][j] += g[k][j] * xh;
+        g[k][j] *= wv[k][j];
+        dot[k] += g[k][j] * xh;
+      }
+      tot += dot[k];
+    }
+    if (per_head) {
+#pragma unroll
+      for (int k = 0; k < VPT; ++k) {
+        for (int o = vph >> 1; o > 0; o >>= 1) dot[k] += __shfl_xor_sync(0xffffffffu, dot[k], o);
+        dot[k] /= (float)D;
+      }
+    } else {
+      tot = warp_sum(tot);
+      float* rd = red[row & 1];
+      if ((threadIdx.x & 31) == 0) rd[threadIdx.x >> 5] = tot;
+      __syncthreads();
+      float t = 0.f;
+#pragma unroll
+      for (int i = 0; i < NTH / 32; ++i) t += rd[i];
+#pragma unroll
+      for (int k = 0; k < VPT; ++k) dot[k] = t / (float)C;
+    }
+#pragma unroll
+    for (int k = 0; k < VPT; ++k) {
+      const int vec = threadIdx.x + k * NTH;
+      if (vec < nvec) {
+        float xv[8], o[8];
+        forget(cx[k]);
+        unpack8(cx[k], xv);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) o[j] = rs[k] * (g[k][j] - xv[j] * rs[k] * dot[k]);
+        store8(dx + (long long)row * lddx + vec * 8, o);
+      }
+    }
+  }
+  if (partial && w) {
+    float* pw = partial + (long long)blockIdx.x * C;
+#pragma unroll
+    for (int k = 0; k < VPT; ++k) {
+      const int vec = threadIdx.x + k * NTH;
+      if (vec < nvec) {
+        *reinterpret_cast<float4*>(pw + vec * 8) = make_float4(acc[k][0], acc[k][1], acc[k][2], acc[k][3]);
+        *reinterpret_cast<float4*>(pw + vec * 8 + 4) = make_float4(acc[k][4], acc[k][5], acc[k][6], acc[k][7]);
+      }
+    }
+  }
+}
+
 // Forward: in = x. Saves rstd ([rows] or [rows, H]) when w != null.
 static int rmsrope_fwd_impl(const void* x, long long ldx, void* y, long long ldy, const float* w,
                             const void* freqs, int freq_rows, float* rstd, int rows, int C, int D,
@@ -795,12 +906,15 @@ static int rmsrope_fwd_impl(const void* x, long long ldx, void* y, long long ldy
   TT_CHECK(freqs == nullptr || (D % 8 == 0 && freq_rows > 0), "rmsrope_fwd: bad rotary table");
   TT_CHECK(ldx % 8 == 0 && ldy % 8 == 0, "rmsrope_fwd: leading dims misaligned");
   TT_CHECK(aligned16(x) && aligned16(y) && aligned16(w) && aligned16(freqs), "rmsrope_fwd: misaligned pointer");
-  if (!per_head && C % 256 == 0 && C <= 2048) {  // one row per warp
+  if (C % 256 == 0 && (C <= 2048 || C == 3072 || C == 5120)) {  // one row per warp
     const int want = (rows + NT / 32 - 1) / (NT / 32);
     const int wgrid = want < 148 * 8 ? want : 148 * 8;
-#define TT_RMS_FWD_WARP(NVV)                                                                                        \
-  rmsrope_fwd_warp_kernel<NVV><<<wgrid, NT, 0, stream>>>((const bf16*)x, ldx, (bf16*)y, ldy, w, (const float2*)freqs, \
-                                                         freq_rows, rstd, rows, D, eps, sc, ssq, ssq_n, ssq_ld)
+#define TT_RMS_FWD_WARP(NVV)                                                                                              \
+  do {                                                                                                                    \
+    auto kern = per_head ? rmsrope_fwd_warp_kernel<NVV, true> : rmsrope_fwd_warp_kernel<NVV, false>;                      \
+    kern<<<wgrid, NT, 0, stream>>>((const bf16*)x, ldx, (bf16*)y, ldy, w, (const float2*)freqs, freq_rows, rstd, rows, D, \
+                                   eps, sc, ssq, ssq_n, ssq_ld);                                                          \
+  } while (0)
     switch (C / 256) {
       case 1: TT_RMS_FWD_WARP(1); break;
       case 2: TT_RMS_FWD_WARP(2); break;
@@ -809,7 +923,9 @@ static int rmsrope_fwd_impl(const void* x, long long ldx, void* y, long long ldy
       case 5: TT_RMS_FWD_WARP(5); break;
       case 6: TT_RMS_FWD_WARP(6); break;
       case 7: TT_RMS_FWD_WARP(7); break;
-      default: TT_RMS_FWD_WARP(8); break;
+      case 8: TT_RMS_FWD_WARP(8); break;
+      case 12: TT_RMS_FWD_WARP(12); break;
+      default: TT_RMS_FWD_WARP(20); break;
     }
 #undef TT_RMS_FWD_WARP
     TT_LAUNCH_CHECK();
@@ -817,9 +933,8 @@ static int rmsrope_fwd_impl(const void* x, long long ldx, void* y, long long ldy
   }
   const int rpc = rows > 148 * 32 ? (rows + 148 * 16 - 1) / (148 * 16) : 1;
   const int grid = (rows + rpc - 1) / rpc;
-  TT_DISPATCH_VPT(vpt_for(C), rmsrope_kernel<VPT, false><<<grid, NT, 0, stream>>>(
-      (const bf16*)x, ldx, nullptr, 0, (bf16*)y, ldy, w, (const float2*)freqs, freq_rows, rstd,
-      nullptr, rows, C, D, per_head, eps, rpc, sc, ssq, ssq_n, ssq_ld));
+  TT_DISPATCH_VPT(vpt_for(C), rmsrope_kernel<VPT><<<grid, NT, 0, stream>>>(
+      (const bf16*)x, ldx, (bf16*)y, ldy, w, (const float2*)freqs, freq_rows, rstd, rows, C, D, per_head, eps, rpc, sc, ssq, ssq_n, ssq_ld));
   TT_LAUNCH_CHECK();
   return 0;
 }
@@ -904,9 +1019,16 @@ TT_API int tt_rmsrope_bwd(const void* dy, long long lddy, const void* x, long lo
     TT_LAUNCH_CHECK();
     return 0;
   }
-  TT_DISPATCH_VPT(vpt_for(C), rmsrope_kernel<VPT, true><<<grid, NT, 0, stream>>>(
-      (const bf16*)dy, lddy, (const bf16*)x, ldx, (bf16*)dx, lddx, w, (const float2*)freqs, freq_rows,
-      rstd, partial, rows, C, D, per_head, 0.f, rpc, TTScatter{}));
+#define TT_RMS_BWD_ROW(V, T, B)                                                                                            \
+  rmsrope_bwd_row_kernel<V, T, B><<<grid, T, 0, stream>>>((const bf16*)dy, lddy, (const bf16*)x, ldx, (bf16*)dx, lddx, w,  \
+                                                       (const float2*)freqs, freq_rows, rstd, partial, rows, C, D,      \
+                                                       per_head, rpc)
+  if (C <= 1536) TT_RMS_BWD_ROW(1, 192, 5);
+  else if (C <= 2048) TT_RMS_BWD_ROW(1, 256, 4);
+  else if (C <= 3072) TT_RMS_BWD_ROW(1, 384, 2);
+  else if (C <= 5120) TT_RMS_BWD_ROW(2, 320, 2);
+  else TT_RMS_BWD_ROW(2, 384, 1);
+#undef TT_RMS_BWD_ROW
   TT_LAUNCH_CHECK();
   return 0;
 }
