@@ -15,8 +15,13 @@
 // cp.async.bulk per ring slot.  A stride-2 window is a 1-stride one over the four pixel phases of its input
 // (tt_blk_move mode 1), each phase with its own taps.
 //
-// Roles (384 threads): warp 0 input boxes, warp 1 weight tiles, warp 2 tensor memory + MMA issue, warps 4..11 epilogue
-// (bias, residual, store).  Every wait is bounded.
+// Roles (384 threads): warp 0 input boxes, warp 1 weight tiles, warps 2 and 3 MMA issue (one 128-row accumulator each;
+// warp 2 also holds the tensor memory), warps 4..11 epilogue (bias, residual, store).  Every wait is bounded.
+//
+// What bounds it: the issuing threads.  An MMA is 48 to 96 clocks, and the wait, fence and commit around a weight tile cost
+// one thread about as much as the tile's MMAs: with a single issuer halving its MMAs took away a fifth of the time, while
+// loading no input, loading no weights, aligning every operand row or padding the weight planes changed nothing.  Two
+// issuers hide each other's waits, and the loop over a weight tile is unrolled.
 #include "tt_common.cuh"
 
 using namespace tt;
@@ -80,6 +85,14 @@ __device__ __forceinline__ void umma_conv(uint32_t d, uint32_t a_lo, uint32_t a_
         "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(acc)
         : "memory");
   }
+}
+// STEPS consecutive 32-byte steps along K
+template <bool F32, int STEPS>
+__device__ __forceinline__ void umma_steps(uint32_t d, uint32_t a_lo, uint32_t a_hi, uint32_t a_step, uint32_t b_lo,
+                                           uint32_t b_hi, uint32_t b_step, uint32_t idesc, uint32_t acc) {
+#pragma unroll
+  for (int k = 0; k < STEPS; ++k)
+    umma_conv<F32>(d, a_lo + k * a_step, a_hi, b_lo + k * b_step, b_hi, idesc, k ? 1u : acc);
 }
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile(
@@ -152,9 +165,9 @@ conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ Con
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n_acc = p.NT <= 128 ? 2 : 1;  // accumulator buffers: 2 x 128 rows x NT columns each, 512 columns in all
   if (threadIdx.x == 0) {
-    for (int i = 0; i < CV_MAX_A; ++i) { mbar_init(&a_full[i], 1); mbar_init(&a_empty[i], 1); }
-    for (int i = 0; i < CV_MAX_B; ++i) { mbar_init(&b_full[i], 1); mbar_init(&b_empty[i], 1); }
-    for (int i = 0; i < 2; ++i) { mbar_init(&tfull[i], 1); mbar_init(&tempty[i], 8); }
+    for (int i = 0; i < CV_MAX_A; ++i) { mbar_init(&a_full[i], 1); mbar_init(&a_empty[i], 2); }
+    for (int i = 0; i < CV_MAX_B; ++i) { mbar_init(&b_full[i], 1); mbar_init(&b_empty[i], 2); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&tfull[i], 2); mbar_init(&tempty[i], 8); }
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -211,8 +224,9 @@ conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ Con
         }
       }
     }
-  } else if (warp == 2) {
+  } else if (warp < 4) {
     if (lane == 0) {  // ---------------------------------------------- MMA issue
+      const int m = warp - 2;
       // bits 7..9 / 10..12: operand formats (1 = bf16, 2 = tf32); fp32 accumulate; both K-major
       const uint32_t fmt = F32 ? 2u : 1u;
       const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(p.NT >> 3) << 17) | (8u << 24);
@@ -231,26 +245,29 @@ conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ Con
         const uint32_t tph = n_acc == 2 ? ((tcount >> 1) & 1) : (tcount & 1);
         if (!mbar_wait(&tempty[buf], tph ^ 1, abort_flag, p.status, TT_ST_TIMEOUT_MMA)) break;
         tc_fence_after();
-        const uint32_t d = tmem_base + buf * 256;
+        const uint32_t d = tmem_base + buf * 256 + m * p.NT;
         uint32_t acc = 0;
         for (int g = 0; g < p.n_groups && ok; ++g) {
           if (at.t * p.t_stride + p.g[g].dt + p.t_off < 0) continue;
           for (int cb = 0; cb < p.n_cb && ok; ++cb) {
             if (!mbar_wait(&a_full[sa], pa, abort_flag, p.status, TT_ST_TIMEOUT_MMA + 1)) { ok = false; break; }
-            const uint32_t a0 = (smem_u32(sA + sa * p.a_slot) >> 4);
+            const uint32_t a0 = (smem_u32(sA + sa * p.a_slot) >> 4) + m * 8;
             for (int tap = 0; tap < p.g[g].n_taps && ok; ++tap) {
               uint32_t ax = a_top | (a0 + p.g[g].off[tap]);
               for (int u = 0; u < per_box; ++u) {
                 if (!mbar_wait(&b_full[sb], pb, abort_flag, p.status, TT_ST_TIMEOUT_MMA + 2)) { ok = false; break; }
                 tc_fence_after();
-                uint32_t bx = b_top | (smem_u32(sB + sb * p.b_bytes) >> 4);
-                for (int k = 0; k < p.UC; k += 2) {
-                  umma_conv<F32>(d, ax, a_hi, bx, b_hi, idesc, acc);
-                  umma_conv<F32>(d + p.NT, ax + 8, a_hi, bx, b_hi, idesc, acc);
-                  acc = 1;
-                  ax += 2 * a_lbo;
-                  bx += 2 * b_lbo;
+                const uint32_t bx = b_top | (smem_u32(sB + sb * p.b_bytes) >> 4);
+                if (p.UC == 12) {
+                  umma_steps<F32, 6>(d, ax, a_hi, 2 * a_lbo, bx, b_hi, 2 * b_lbo, idesc, acc);
+                } else if (p.UC == 6) {
+                  umma_steps<F32, 3>(d, ax, a_hi, 2 * a_lbo, bx, b_hi, 2 * b_lbo, idesc, acc);
+                } else {
+                  for (int k = 0; k < p.UC; k += 2)
+                    umma_steps<F32, 1>(d, ax + k * a_lbo, a_hi, 0, bx + k * b_lbo, b_hi, 0, idesc, k ? 1u : acc);
                 }
+                acc = 1;
+                ax += p.UC * a_lbo;
                 tc_commit(&b_empty[sb]);
                 if (++sb == p.b_stages) { sb = 0; pb ^= 1; }
               }
@@ -339,10 +356,17 @@ struct PackParams {
 };
 template <bool F32>
 __global__ void __launch_bounds__(256)
-conv_pack_kernel(const void* __restrict__ src, void* __restrict__ dst, const PackParams p, long long chunks_per_tile) {
+conv_pack_kernel(const void* __restrict__ src, const void* __restrict__ bias, void* __restrict__ dst, const PackParams p,
+                 long long chunks_per_tile) {
   constexpr int E = Chunk<F32>::E;
   const long long i = (long long)blockIdx.x * 256 + threadIdx.x;  // one 16-byte chunk of one output channel
-  if (i >= chunks_per_tile * p.n_tiles * p.NT) return;
+  const long long total = chunks_per_tile * p.n_tiles * p.NT;
+  if (i < p.n_tiles * p.NT) {  // the bias follows the weights, in fp32
+    float b = 0.f;
+    if (bias && i < p.N_real) b = F32 ? reinterpret_cast<const float*>(bias)[i] : __bfloat162float(reinterpret_cast<const bf16*>(bias)[i]);
+    reinterpret_cast<float*>(reinterpret_cast<uint4*>(dst) + total)[i] = b;
+  }
+  if (i >= total) return;
   const int n = (int)(i % p.NT);
   long long r = i / p.NT;
   const int nt = (int)(r / chunks_per_tile);
@@ -372,7 +396,7 @@ conv_pack_kernel(const void* __restrict__ src, void* __restrict__ dst, const Pac
 // hold consecutive pixels, so every access is a full 512-byte row of a plane.
 template <bool F32, int NCH>
 __global__ void __launch_bounds__(256)
-chan_norm_kernel(const uint4* __restrict__ x, uint4* __restrict__ y, const float* __restrict__ gamma, long long hw,
+chan_norm_kernel(const uint4* __restrict__ x, uint4* __restrict__ y, const void* __restrict__ gamma, long long hw,
                  int chunks, float scale, int act) {
   constexpr int E = Chunk<F32>::E;
   __shared__ float red[4][64];
@@ -404,11 +428,12 @@ chan_norm_kernel(const uint4* __restrict__ x, uint4* __restrict__ y, const float
   for (int k = 0; k < NCH; ++k) {
     const int c = sl + 4 * k;
     if (c < chunks) {
-      float f[E];
+      float f[E], g[E];
       Chunk<F32>::get(v[k], f);
+      Chunk<F32>::get(reinterpret_cast<const uint4*>(gamma)[c], g);
 #pragma unroll
       for (int j = 0; j < E; ++j) {
-        float t = f[j] * inv * gamma[c * E + j];
+        float t = f[j] * inv * g[j];
         if (act) t = t / (1.f + (F32 ? expf(-t) : __expf(-t)));
         f[j] = F32 ? round_tf32(t) : t;
       }
@@ -504,14 +529,11 @@ int largest_even_divisor(int n, int cap) {
   return 0;
 }
 struct ConvShape { int NT, KC, UC, n_cb, n_tiles; };
-// How a convolution of `chunks` input chunks (per tap) and N output channels (both padded) is cut: as many output
-// channels per tile as 192 (two accumulators of 128 rows fit tensor memory twice up to 128, once up to 256 columns),
-// boxes of up to 12 chunks (62 KB, two in flight), weight tiles of at most 18 KB.
-int conv_shape(int chunks, int N, ConvShape* s) {
-  if (chunks < 2 || chunks % 2 || N < 16 || N % 16) return -1;
-  int nt = N < 192 ? N : 192;
-  while (nt >= 16 && N % nt) nt -= 16;
-  if (nt < 16) return -1;
+// How a convolution of `chunks` input chunks (per tap) and N output channels (both padded) is cut: NT output channels per
+// tile (two accumulators of 128 rows fit tensor memory twice up to 128, once up to 256 columns), boxes of up to 12
+// chunks (62 KB, two in flight), weight tiles of at most 18 KB.
+int conv_shape(int chunks, int N, int nt, ConvShape* s) {
+  if (chunks < 2 || chunks % 2 || N < 16 || N % 16 || nt < 16 || nt > 192 || nt % 16 || N % nt) return -1;
   s->NT = nt;
   s->n_tiles = N / nt;
   s->KC = largest_even_divisor(chunks, 12);
@@ -546,17 +568,34 @@ int conv_groups(int kind, int kt, int chunks, int box_w, ConvGroup* g, int tap_i
 
 }  // namespace
 
-// Bytes of the packed weights, or -1 when the shape is outside the kernel's domain (kt <= 4).
-TT_API long long tt_conv_packed_bytes(int kind, int kt, int chunks, int N) {
-  ConvShape s;
-  if (kind < 0 || kind > 2 || kt < 1 || kt > 4 || conv_shape(chunks, N, &s)) return -1;
-  return (long long)(kind == 2 ? 9 : (kind == 0 ? 9 : 1) * kt) * chunks * N * 16;
+// Output channels per tile for `frames` x H x W output pixels: the widest divisor of N whose waves over the SMs, times
+// the cost of a wave, are fewest.  Measured with 384 channels, a wave of tiles wider than 96 takes 75 us, a wave of 96
+// down to 16 takes 50 (the issue of an MMA bounds the narrow ones), so 96 pays where 192 would leave SMs idle:
+// 3 x 30 x 52 pixels are 48 tiles of 192 (91.8 us) or 96 tiles of 96 (70.6 us); 5 x 120 x 208 take 604 and 772 us.
+TT_API int tt_conv_tile_channels(int N, int frames, int H, int W, int sms) {
+  if (N < 16 || N % 16 || frames < 1 || H < 1 || W < 1 || sms < 1) return -1;
+  const long long pix = (long long)((W + CV_TW - 1) / CV_TW) * ((H + CV_TH - 1) / CV_TH) * frames;
+  int best = -1;
+  double cost = 0;
+  for (int nt = 192; nt >= 16; nt -= 16) {
+    if (N % nt) continue;
+    const long long waves = (pix * (N / nt) + sms - 1) / sms;
+    const double c = (double)waves * (nt > 96 ? 75 : 50);
+    if (best < 0 || c < cost) { best = nt; cost = c; }
+  }
+  return best;
 }
 
-TT_API int tt_conv_pack(const void* w, int f32, int kind, int kt, int C_real, int N_real, int chunks, int N, void* dst,
-                        cudaStream_t stream) {
+// Bytes of the packed weights and bias, or -1 when the shape is outside the kernel's domain (kt <= 4).
+TT_API long long tt_conv_packed_bytes(int kind, int kt, int chunks, int N) {
+  if (kind < 0 || kind > 2 || kt < 1 || kt > 4 || chunks < 2 || chunks % 2 || N < 16 || N % 16) return -1;
+  return (long long)(kind == 2 ? 9 : (kind == 0 ? 9 : 1) * kt) * chunks * N * 16 + (long long)N * 4;
+}
+
+TT_API int tt_conv_pack(const void* w, const void* bias, int f32, int kind, int kt, int C_real, int N_real, int chunks,
+                        int N, int nt, void* dst, cudaStream_t stream) {
   ConvShape s;
-  TT_CHECK(tt_conv_packed_bytes(kind, kt, chunks, N) > 0 && !conv_shape(chunks, N, &s), "conv_pack: bad shape");
+  TT_CHECK(tt_conv_packed_bytes(kind, kt, chunks, N) > 0 && !conv_shape(chunks, N, nt, &s), "conv_pack: bad shape");
   TT_CHECK(N_real <= N && C_real <= chunks * (f32 ? 4 : 8) && ((uintptr_t)dst & 15) == 0, "conv_pack: bad arguments");
   ConvGroup g[4];
   PackParams p;
@@ -566,8 +605,8 @@ TT_API int tt_conv_pack(const void* w, int f32, int kind, int kt, int C_real, in
   for (int i = 0; i < p.n_groups; ++i) { p.n_taps[i] = g[i].n_taps; p.taps_total += g[i].n_taps; }
   const long long per_tile = (long long)p.taps_total * chunks, total = per_tile * N;
   const unsigned grid = (unsigned)((total + 255) / 256);
-  if (f32) conv_pack_kernel<true><<<grid, 256, 0, stream>>>(w, dst, p, per_tile);
-  else conv_pack_kernel<false><<<grid, 256, 0, stream>>>(w, dst, p, per_tile);
+  if (f32) conv_pack_kernel<true><<<grid, 256, 0, stream>>>(w, bias, dst, p, per_tile);
+  else conv_pack_kernel<false><<<grid, 256, 0, stream>>>(w, bias, dst, p, per_tile);
   TT_LAUNCH_CHECK();
   return 0;
 }
@@ -575,14 +614,14 @@ TT_API int tt_conv_pack(const void* w, int f32, int kind, int kt, int C_real, in
 // x: [T_in][x_chunks][H_in][W_in][E] (kind 2: x_chunks = 4 * chunks pixel phases).  Output frame t reads input frames
 // t * t_stride + t_off + (0 .. kt - 1); frames below zero are zeros.  Output pixels H x W.
 TT_API int tt_conv(const void* x, int f32, int kind, int kt, int T_in, int H_in, int W_in, int chunks, const void* packed,
-                   int N, const float* bias, void* out, const void* res, int T, int H, int W, int t_stride, int t_off,
+                   int N, int nt, void* out, const void* res, int T, int H, int W, int t_stride, int t_off,
                    int C_out, int t_mul, int planar, int C_real, unsigned* status, cudaStream_t stream) {
   ConvShape s;
-  TT_CHECK(kind >= 0 && kind <= 2 && kt >= 1 && kt <= 4 && (kind != 2 || kt == 1) && !conv_shape(chunks, N, &s),
+  TT_CHECK(kind >= 0 && kind <= 2 && kt >= 1 && kt <= 4 && (kind != 2 || kt == 1) && !conv_shape(chunks, N, nt, &s),
            "conv: bad shape kind=%d kt=%d chunks=%d N=%d", kind, kt, chunks, N);
   TT_CHECK(T > 0 && H > 0 && W > 0 && T_in > 0 && H_in > 0 && W_in > 0, "conv: empty input or output");
   TT_CHECK((long long)(T - 1) * t_stride + kt - 1 + t_off < T_in && kt - 1 + t_off >= 0, "conv: frames out of range");
-  TT_CHECK((((uintptr_t)x | (uintptr_t)packed | (uintptr_t)out | (uintptr_t)res | (uintptr_t)bias) & 15) == 0,
+  TT_CHECK((((uintptr_t)x | (uintptr_t)packed | (uintptr_t)out | (uintptr_t)res) & 15) == 0,
            "conv: operands must be 16-byte aligned");
   TT_CHECK(planar || (C_out > 0 && C_out % 16 == 0 && N % C_out == 0), "conv: bad output channel split");
   const int E = f32 ? 4 : 8;
@@ -613,7 +652,8 @@ TT_API int tt_conv(const void* x, int f32, int kind, int kt, int T_in, int H_in,
   for (int i = 0; i < p.n_groups; ++i) taps += p.g[i].n_taps;
   p.B = (const uint8_t*)packed;
   p.b_tile_bytes = (long long)taps * chunks * s.NT * 16;
-  p.bias = bias; p.out = out; p.res = res;
+  p.bias = reinterpret_cast<const float*>(p.B + p.b_tile_bytes * s.n_tiles);
+  p.out = out; p.res = res;
   p.C_out = C_out; p.t_mul = t_mul; p.planar = planar; p.C_real = C_real; p.status = status;
   CUtensorMap tm;
   const int xc = kind == 2 ? 4 * chunks : chunks;
@@ -632,10 +672,11 @@ TT_API int tt_conv(const void* x, int f32, int kind, int kt, int T_in, int H_in,
   return 0;
 }
 
-TT_API int tt_chan_norm(const void* x, void* y, const float* gamma, int f32, int frames, int chunks, long long hw,
+// gamma: [C] in the type of x
+TT_API int tt_chan_norm(const void* x, void* y, const void* gamma, int f32, int frames, int chunks, long long hw,
                         int act, cudaStream_t stream) {
   TT_CHECK(frames > 0 && frames < 65536 && hw > 0 && chunks > 0 && chunks <= 96, "chan_norm: bad shape");
-  TT_CHECK((((uintptr_t)x | (uintptr_t)y) & 15) == 0, "chan_norm: misaligned");
+  TT_CHECK((((uintptr_t)x | (uintptr_t)y | (uintptr_t)gamma) & 15) == 0, "chan_norm: misaligned");
   const dim3 grid((unsigned)((hw + 63) / 64), frames);
   const float scale = sqrtf((float)(chunks * (f32 ? 4 : 8)));
 #define TT_NORM(F, N) chan_norm_kernel<F, N><<<grid, 256, 0, stream>>>((const uint4*)x, (uint4*)y, gamma, hw, chunks, scale, act)

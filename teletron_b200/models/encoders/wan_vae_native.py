@@ -62,17 +62,11 @@ class Run:
     def __init__(self):
         self.packs = {}
 
-    def pack(self, m, kind):
+    def conv(self, m, kind, x, frames, hw, **kw):
         pk = self.packs.get(m)
         if pk is None:
-            pk = self.packs[m] = C.PackedConv(m.weight, m.bias, kind)
-        return pk
-
-    def gamma(self, m):
-        g = self.packs.get(m)
-        if g is None:
-            g = self.packs[m] = m.gamma.detach().float().reshape(-1).contiguous()
-        return g
+            pk = self.packs[m] = C.PackedConv(m.weight, m.bias, kind, (frames, *hw))
+        return C.conv(x, pk, frames, hw, **kw)
 
     # -------------------------------------------------------------------------------------------------- pieces
     def _with_history(self, m, shape, like):
@@ -95,9 +89,9 @@ class Run:
 
     def norm_conv(self, norm, m, x, res=None, planar=False):
         buf, view, t_off = self._with_history(m, x.shape, x)
-        C.chan_norm(x, self.gamma(norm), view)
+        C.chan_norm(x, norm.gamma.detach().reshape(-1), view)
         self._keep_history(m, buf)
-        return C.conv(buf, self.pack(m, C.CONV_SPATIAL), x.shape[0], x.shape[2:4], t_off=t_off, res=res, planar=planar)
+        return self.conv(m, C.CONV_SPATIAL, buf, x.shape[0], x.shape[2:4], t_off=t_off, res=res, planar=planar)
 
     def first_conv(self, m, x):
         """x: planar [C, T, H, W]."""
@@ -107,7 +101,7 @@ class Run:
         if st is not None and st.get(m) is not None:
             x, t_off = torch.cat([st[m], x]), 0
         self._keep_history(m, x)
-        return C.conv(x, self.pack(m, C.CONV_SPATIAL), frames, x.shape[2:4], t_off=t_off)
+        return self.conv(m, C.CONV_SPATIAL, x, frames, x.shape[2:4], t_off=t_off)
 
     def res_block(self, m, x):
         r = m.residual
@@ -115,7 +109,7 @@ class Run:
         if isinstance(m.shortcut, nn.Identity):
             skip = x
         else:
-            skip = C.conv(C.rounded(x), self.pack(m.shortcut, C.CONV_POINT), x.shape[0], x.shape[2:4])
+            skip = self.conv(m.shortcut, C.CONV_POINT, C.rounded(x), x.shape[0], x.shape[2:4])
         return self.norm_conv(r[3], r[6], h, res=skip)
 
     def attention(self, m, x):
@@ -127,7 +121,7 @@ class Run:
         if st is not None:
             st[("seen", m)] = True
         hw = (x.shape[2] // 2, x.shape[3] // 2)
-        x = C.conv(C.phases2(x), self.pack(m.resample[1], C.CONV_STRIDE2), x.shape[0], hw)
+        x = self.conv(m.resample[1], C.CONV_STRIDE2, C.phases2(x), x.shape[0], hw)
         if m.mode != "downsample3d":
             return x
         last = x[-1:].clone() if st is not None else None
@@ -141,7 +135,7 @@ class Run:
             out = torch.empty((keep + n, *x.shape[1:]), dtype=x.dtype, device=x.device)
             if keep:
                 out[0].copy_(x[0])
-            C.conv(C.rounded(x), self.pack(m.time_conv, C.CONV_POINT), n, hw, t_stride=2, out=out[keep:])
+            self.conv(m.time_conv, C.CONV_POINT, C.rounded(x), n, hw, t_stride=2, out=out[keep:])
             x = out
         if st is not None:
             st[("last", m)] = last
@@ -163,9 +157,9 @@ class Run:
                 out = torch.empty((keep + 2 * (t - keep), *x.shape[1:]), dtype=x.dtype, device=x.device)
                 if keep:
                     out[0].copy_(x[0])
-                C.conv(buf, self.pack(m.time_conv, C.CONV_POINT), t - keep, hw, t_off=t_off, out=out[keep:], t_mul=2)
+                self.conv(m.time_conv, C.CONV_POINT, buf, t - keep, hw, t_off=t_off, out=out[keep:], t_mul=2)
                 x = out
-        return C.conv(C.enlarge2(x), self.pack(m.resample[1], C.CONV_SPATIAL), x.shape[0], (2 * hw[0], 2 * hw[1]))
+        return self.conv(m.resample[1], C.CONV_SPATIAL, C.enlarge2(x), x.shape[0], (2 * hw[0], 2 * hw[1]))
 
     # ------------------------------------------------------------------------------------------------- networks
     def _layers(self, layers, x):

@@ -6,7 +6,6 @@ cuDNN does with them by default; the operands are rounded to nearest, not trunca
 from __future__ import annotations
 
 import torch
-import torch.nn.functional as F
 
 from . import _lib
 
@@ -22,10 +21,11 @@ def chunk_elems(dtype) -> int:
 
 
 class PackedConv:
-    """Weights of one convolution in the order the kernel reads them, and the bias in fp32; channels are padded to
-    an even number of chunks (inputs) and to 16 (outputs)."""
+    """Weights and bias of one convolution in the order the kernel reads them; channels are padded to an even number of
+    chunks (inputs) and to 16 (outputs).  ``size`` is the (frames, height, width) of the output that the split into
+    output-channel tiles is made for; other sizes are computed with it too."""
 
-    def __init__(self, weight: torch.Tensor, bias, kind: int):
+    def __init__(self, weight: torch.Tensor, bias, kind: int, size):
         n, c = weight.shape[:2]
         self.kind, self.kt = kind, (weight.shape[2] if weight.dim() == 5 else 1)
         e = chunk_elems(weight.dtype)
@@ -33,16 +33,17 @@ class PackedConv:
         L = _lib.lib()
         L.tt_conv_packed_bytes.restype = _lib.c_ll
         dims = (_lib.c_int(kind), _lib.c_int(self.kt))
-        size = L.tt_conv_packed_bytes(*dims, _lib.c_int(self.chunks), _lib.c_int(self.n))
-        if size < 0:
+        nbytes = L.tt_conv_packed_bytes(*dims, _lib.c_int(self.chunks), _lib.c_int(self.n))
+        if nbytes < 0:
             raise ValueError(f"convolution outside the kernel's domain: weight {tuple(weight.shape)}")
-        self.data = torch.empty(size, dtype=torch.uint8, device=weight.device)
+        self.nt = L.tt_conv_tile_channels(_lib.c_int(self.n), *(_lib.c_int(v) for v in size), _lib.c_int(L.tt_num_sms()))
+        self.data = torch.empty(nbytes, dtype=torch.uint8, device=weight.device)
         w = weight.detach().contiguous()
-        _lib.check(L.tt_conv_pack(_lib.ptr(w), _lib.c_int(_f32(w.dtype)), *dims, _lib.c_int(c), _lib.c_int(n),
-                                  _lib.c_int(self.chunks), _lib.c_int(self.n), _lib.ptr(self.data), _lib.stream()),
-                   "tt_conv_pack")
-        b = torch.zeros(n, device=w.device) if bias is None else bias.detach().float()
-        self.bias = F.pad(b, (0, self.n - n)).contiguous()
+        b = None if bias is None else bias.detach().contiguous()
+        assert b is None or (b.dtype == w.dtype and b.device == w.device and b.numel() == n)
+        _lib.check(L.tt_conv_pack(_lib.ptr(w), _lib.ptr(b), _lib.c_int(_f32(w.dtype)), *dims, _lib.c_int(c), _lib.c_int(n),
+                                  _lib.c_int(self.chunks), _lib.c_int(self.n), _lib.c_int(self.nt), _lib.ptr(self.data),
+                                  _lib.stream()), "tt_conv_pack")
 
 
 def conv(x: torch.Tensor, pk: PackedConv, frames: int, hw, *, t_stride=1, t_off=0, out=None, res=None, t_mul=1,
@@ -65,16 +66,17 @@ def conv(x: torch.Tensor, pk: PackedConv, frames: int, hw, *, t_stride=1, t_off=
     _lib.check(_lib.lib().tt_conv(
         _lib.ptr(x), _lib.c_int(_f32(x.dtype)), _lib.c_int(pk.kind), _lib.c_int(pk.kt), _lib.c_int(x.shape[0]),
         _lib.c_int(x.shape[2]), _lib.c_int(x.shape[3]), _lib.c_int(pk.chunks), _lib.ptr(pk.data), _lib.c_int(pk.n),
-        _lib.ptr(pk.bias), _lib.ptr(out), _lib.ptr(res), _lib.c_int(frames), _lib.c_int(h), _lib.c_int(w),
+        _lib.c_int(pk.nt), _lib.ptr(out), _lib.ptr(res), _lib.c_int(frames), _lib.c_int(h), _lib.c_int(w),
         _lib.c_int(t_stride), _lib.c_int(t_off), _lib.c_int(c_out), _lib.c_int(t_mul), _lib.c_int(int(planar)),
         _lib.c_int(pk.n_real), _lib.ptr(_lib.status_word(x.device)), _lib.stream()), "tt_conv")
     return out
 
 
 def chan_norm(x: torch.Tensor, gamma: torch.Tensor, out: torch.Tensor, act: bool = True) -> torch.Tensor:
-    """``silu(x / max(|x|, 1e-12) * sqrt(C) * gamma)`` over the channels of every pixel; gamma fp32 [C]."""
+    """``silu(x / max(|x|, 1e-12) * sqrt(C) * gamma)`` over the channels of every pixel; gamma [C] in x's type."""
     t, chunks, h, w, e = x.shape
     assert x.is_contiguous() and out.is_contiguous() and out.shape == x.shape and gamma.numel() == chunks * e
+    assert gamma.dtype == x.dtype and gamma.is_contiguous()
     _lib.check(_lib.lib().tt_chan_norm(_lib.ptr(x), _lib.ptr(out), _lib.ptr(gamma), _lib.c_int(_f32(x.dtype)),
                                        _lib.c_int(t), _lib.c_int(chunks), _lib.c_ll(h * w), _lib.c_int(int(act)),
                                        _lib.stream()), "tt_chan_norm")

@@ -31,7 +31,7 @@ def test_causal_conv(dtype, ci, co, t, h, w):
     torch.manual_seed(0)
     x, k, b = _rand(ci, t, h, w, dtype=dtype), _rand(co, ci, 3, 3, 3, dtype=dtype, scale=(27 * ci) ** -0.5), _rand(co, dtype=dtype)
     ref = F.conv3d(F.pad(x.double()[None], (1, 1, 1, 1, 2, 0)), k.double(), b.double())[0]
-    xb, pk = C.from_planar(x, True), C.PackedConv(k, b, C.CONV_SPATIAL)
+    xb, pk = C.from_planar(x, True), C.PackedConv(k, b, C.CONV_SPATIAL, (t, h, w) if w % 2 else (t, 480, 832))
     if co % 16:
         y = C.conv(xb, pk, t, (h, w), t_off=-2, planar=True)
     else:
@@ -53,16 +53,16 @@ def test_resampling_convs(dtype, h, w):
     xb, xd = C.from_planar(x, True), x.double()
     k = _rand(c, c, 3, 3, dtype=dtype, scale=(9 * c) ** -0.5)
     ref = F.conv2d(F.pad(xd.transpose(0, 1), (0, 1, 0, 1)), k.double(), b.double(), stride=2).transpose(0, 1)
-    _close(C.to_planar(C.conv(C.phases2(xb), C.PackedConv(k, b, C.CONV_STRIDE2), t, (h // 2, w // 2))), ref, dtype)
+    _close(C.to_planar(C.conv(C.phases2(xb), C.PackedConv(k, b, C.CONV_STRIDE2, (t, h // 2, w // 2)), t, (h // 2, w // 2))), ref, dtype)
     ref = F.conv2d(F.interpolate(xd.transpose(0, 1), scale_factor=2.0, mode="nearest-exact"), k.double(), b.double(), padding=1)
-    _close(C.to_planar(C.conv(C.enlarge2(xb), C.PackedConv(k, b, C.CONV_SPATIAL), t, (2 * h, 2 * w))), ref.transpose(0, 1), dtype)
+    _close(C.to_planar(C.conv(C.enlarge2(xb), C.PackedConv(k, b, C.CONV_SPATIAL, (t, 2 * h, 2 * w)), t, (2 * h, 2 * w))), ref.transpose(0, 1), dtype)
     k, b2 = _rand(2 * c, c, 3, 1, 1, dtype=dtype, scale=(3 * c) ** -0.5), _rand(2 * c, dtype=dtype)
     ref = F.conv3d(F.pad(xd[None], (0, 0, 0, 0, 2, 0)), k.double(), b2.double())[0].reshape(2, c, t, h, w)
-    y = C.conv(xb, C.PackedConv(k, b2, C.CONV_POINT), t, (h, w), t_off=-2, t_mul=2)
+    y = C.conv(xb, C.PackedConv(k, b2, C.CONV_POINT, (t, h, w)), t, (h, w), t_off=-2, t_mul=2)
     _close(C.to_planar(y), ref.permute(1, 2, 0, 3, 4).reshape(c, 2 * t, h, w), dtype)
     k = _rand(c, c, 3, 1, 1, dtype=dtype, scale=(3 * c) ** -0.5)
     ref = F.conv3d(xd[None], k.double(), b.double(), stride=(2, 1, 1))[0]
-    _close(C.to_planar(C.conv(xb, C.PackedConv(k, b, C.CONV_POINT), 1, (h, w), t_stride=2)), ref, dtype)
+    _close(C.to_planar(C.conv(xb, C.PackedConv(k, b, C.CONV_POINT, (1, h, w)), 1, (h, w), t_stride=2)), ref, dtype)
     _lib.check_status()
 
 
@@ -70,7 +70,7 @@ def test_resampling_convs(dtype, h, w):
 @pytest.mark.parametrize("c", [16, 96, 192, 384])
 def test_chan_norm(dtype, c):
     torch.manual_seed(2)
-    x, g = _rand(c, 2, 13, 11, dtype=dtype), torch.rand(c, device="cuda") + 0.5
+    x, g = _rand(c, 2, 13, 11, dtype=dtype), (torch.rand(c, device="cuda") + 0.5).to(dtype)
     x[:, 0, 0, 0] = 0                                         # a pixel without a direction
     xb = C.from_planar(x)
     y = C.to_planar(C.chan_norm(xb, g, torch.empty_like(xb)))
