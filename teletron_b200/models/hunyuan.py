@@ -93,8 +93,8 @@ class TimestepEmbedder(nn.Module):
         self.linear_2 = nn.Linear(dim, dim)
 
     def forward(self, x):
-        x = F.linear(x.float(), self.linear_1.weight.float(), self.linear_1.bias.float())
-        return F.linear(F.silu(x), self.linear_2.weight.float(), self.linear_2.bias.float())
+        x = ops.row_linear(x, self.linear_1.weight, self.linear_1.bias)
+        return ops.row_linear(F.silu(x), self.linear_2.weight, self.linear_2.bias)
 
 
 class CombinedEmbeddings(nn.Module):
@@ -151,6 +151,10 @@ class FeedForward(nn.Module):
     def forward(self, x_rows):
         h = self.net[0].proj(x_rows, act=self.act)
         return self.net[2](h)
+
+    def residual(self, x_rows, residual, gate, rows_per_batch):
+        """residual + gate * forward(x_rows), in the second projection's epilogue where it ends in no reduce-scatter."""
+        return _project_out(self.net[2], self.net[0].proj(x_rows, act=self.act), residual, gate, rows_per_batch)
 
 
 # ------------------------------------------------------------------------------ token refiner
@@ -341,7 +345,7 @@ class AdaNormZero(nn.Module):
         self.n = n
 
     def forward(self, temb):
-        e = F.linear(F.silu(temb.float()), self.linear.weight.float(), self.linear.bias.float())
+        e = ops.row_linear(F.silu(temb.float()), self.linear.weight, self.linear.bias)
         return e.unflatten(1, (self.n, -1))  # [B, n, C] fp32
 
 
@@ -367,8 +371,8 @@ class DualStreamBlock(nn.Module):
         xt = _project_out(self.attn.to_add_out, ot.reshape(-1, ot.shape[2] * ot.shape[3]), xt, et[:, 2], rt)
         hv, xv = ops.adaln_res(xv, ev[:, 4], ev[:, 3], rv, self.eps)
         ht, xt = ops.adaln_res(xt, et[:, 4], et[:, 3], rt, self.eps)
-        xv = _gated_residual(self.ff(hv), xv, ev[:, 5], rv)
-        xt = _gated_residual(self.ff_context(ht), xt, et[:, 5], rt)
+        xv = self.ff.residual(hv, xv, ev[:, 5], rv)
+        xt = self.ff_context.residual(ht, xt, et[:, 5], rt)
         return xv, xt
 
 
@@ -519,7 +523,7 @@ class HunyuanVideoModel(nn.Module):
         packed = rc.run_blocks([_PairBlock(b) for b in self.transformer_blocks], packed, extra, cfg, self.training)
         packed = rc.run_blocks([_PairBlock(b) for b in self.single_transformer_blocks], packed, extra, cfg, self.training)
         xv = packed[:n_v]
-        e = F.linear(F.silu(temb), self.norm_out.linear.weight.float(), self.norm_out.linear.bias.float())
+        e = ops.row_linear(F.silu(temb), self.norm_out.linear.weight, self.norm_out.linear.bias)
         e = e.unflatten(1, (2, C))  # scale, shift
         rows_per_batch = xv.shape[0] // B
         h = ops.adaln(xv.contiguous(), e[:, 0], e[:, 1], rows_per_batch, cfg.eps)

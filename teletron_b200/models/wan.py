@@ -419,7 +419,7 @@ class WanModel(nn.Module):
         """Tiny per-sample MLPs (time embedding / projection) in fp32."""
         for m in seq:
             if isinstance(m, nn.Linear):
-                x = F.linear(x, m.weight.float(), m.bias.float())
+                x = ops.row_linear(x, m.weight, m.bias)
             else:
                 x = m(x)
         return x

@@ -3,6 +3,7 @@
 ``linear(x, w, b, act)``            y = act(x w^T + b)            act in {None, "gelu", "silu"}
 ``linear_residual(x, w, b, res, gate, rows_per_gate)``
                                     y = res + gate[row // rows_per_gate] * (x w^T + b)
+``row_linear(x, w, b)``              fp32 result for one to four rows
 ``ffn(x, w1, b1, w2, b2, res, gate, rows_per_gate, act)``
                                     the two composed
 
@@ -184,3 +185,65 @@ def ffn(x, w1, b1, w2, b2, res, gate=None, rows_per_gate=1, act="gelu"):
     """res + gate * (act(x @ w1.T + b1) @ w2.T + b2): the feed-forward branch of a DiT block
     (teletron/models/wan/wan_model.py:219-223, 264-265 in the reference)."""
     return linear_residual(linear(x, w1, b1, act), w2, b2, res, gate, rows_per_gate)
+
+
+_ROWLIN_MAX = 4
+_ROWLIN_CHUNKS = 148
+
+
+class _RowLinear(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x, w, b):
+        B, (N, K) = x.shape[0], w.shape
+        x = x.contiguous()
+        y = torch.empty((B, N), dtype=torch.float32, device=x.device)
+        _lib.check(_lib.lib().tt_rowlin_fwd(_lib.ptr(x), _lib.ptr(w), _lib.ptr(b), _lib.ptr(y), _lib.c_int(B), _lib.c_int(N),
+                                            _lib.c_int(K), _lib.stream()), "tt_rowlin_fwd")
+        ctx.save_for_backward(x, w)
+        ctx.w_param, ctx.bias_dtype = w, (None if b is None else b.dtype)
+        return y
+
+    @staticmethod
+    def backward(ctx, dy):
+        x, w = ctx.saved_tensors
+        dy = dy.contiguous()
+        B, (N, K) = x.shape[0], w.shape
+        L = _lib.lib()
+        dims = (_lib.c_int(B), _lib.c_int(N), _lib.c_int(K))
+        dx = dw = db = None
+        if ctx.needs_input_grad[0]:
+            chunks = min(_ROWLIN_CHUNKS, N)
+            partial = torch.empty((chunks, B, K), dtype=torch.float32, device=x.device)
+            dx = torch.empty((B, K), dtype=torch.float32, device=x.device)
+            _lib.check(L.tt_rowlin_dgrad(_lib.ptr(dy), _lib.ptr(w), _lib.ptr(partial), _lib.c_int(chunks), *dims,
+                                         _lib.stream()), "tt_rowlin_dgrad")
+            _lib.check(L.tt_colsum_partials(_lib.ptr(partial), _lib.ptr(dx), _lib.c_int(1), _lib.c_int(chunks),
+                                            _lib.c_int(B * K), _lib.c_int(0), _lib.stream()), "tt_colsum_partials")
+        if ctx.needs_input_grad[1]:
+            owner = ctx.w_param
+            mg = getattr(owner, "main_grad", None)
+            into_main = mg is not None and mg.dtype == torch.float32 and mg.is_contiguous() and mg.data_ptr() % 16 == 0
+            dw = mg if into_main else torch.empty((N, K), dtype=torch.bfloat16, device=x.device)
+            _lib.check(L.tt_rowlin_wgrad(_lib.ptr(dy), _lib.ptr(x), _lib.ptr(dw), _lib.c_int(int(into_main)), *dims,
+                                         _lib.stream()), "tt_rowlin_wgrad")
+            if into_main:
+                dw = None
+                owner.grad_written = True
+                ready = getattr(owner, "grad_ready", None)
+                if ready is not None:
+                    ready()
+        if ctx.bias_dtype is not None and ctx.needs_input_grad[2]:
+            db = dy.sum(0).to(ctx.bias_dtype)
+        return dx, dw, db
+
+
+def row_linear(x, w, b=None):
+    """x @ w.T + b in fp32 for a few rows (timestep embedders, modulation projections).  One to four rows with dense bf16
+    weights on a GPU run the kernels of csrc/rowlin.cu, which read the weights as they are; the rest is F.linear on
+    fp32 copies."""
+    if (x.is_cuda and x.dim() == 2 and 1 <= x.shape[0] <= _ROWLIN_MAX and w.dim() == 2 and w.dtype == torch.bfloat16
+            and x.shape[1] == w.shape[1] and w.shape[1] % 8 == 0 and w.is_contiguous() and w.data_ptr() % 16 == 0
+            and x.device == w.device and (b is None or (b.dtype == torch.bfloat16 and b.is_contiguous()))
+            and not torch.is_autocast_enabled("cuda")):
+        return _RowLinear.apply(x.float(), w, b)
+    return F.linear(x.float(), w.float(), None if b is None else b.float())
