@@ -238,7 +238,7 @@ TT_API int tt_gemm_bf16(const void* A, long long lda, int a_mn, const void* B, l
   TT_CHECK(((uintptr_t)C & 15) == 0, "gemm: C is not 16-byte aligned");
   TT_CHECK(epi >= 0 && epi <= EPI_LAST, "gemm: unknown epilogue %d", epi);
   if (epi == EPI_GATE_RES) {
-    TT_CHECK(residual && gate && rows_per_gate > 0, "gemm: gate/residual epilogue needs both tensors");
+    TT_CHECK(residual && rows_per_gate > 0, "gemm: gate/residual epilogue needs a residual");  // no gate: 1
     TT_CHECK(ldr % 8 == 0 && gate_ld % 4 == 0, "gemm: residual/gate leading dims misaligned");
     TT_CHECK((((uintptr_t)residual | (uintptr_t)gate) & 15) == 0, "gemm: residual/gate misaligned");
   }

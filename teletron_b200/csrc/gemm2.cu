@@ -328,7 +328,7 @@ TT_API int tt_gemm2_bf16(const void* A, long long lda, int a_mn, const void* B, 
   TT_CHECK(ldc % (c_fp32 ? 4 : 8) == 0 && ((uintptr_t)C & 15) == 0, "gemm2: C misaligned");
   TT_CHECK(epi >= 0 && epi <= EPI_LAST, "gemm2: unknown epilogue %d", epi);
   if (epi == EPI_GATE_RES) {
-    TT_CHECK(residual && gate && rows_per_gate > 0, "gemm2: gate/residual epilogue needs both tensors");
+    TT_CHECK(residual && rows_per_gate > 0, "gemm2: gate/residual epilogue needs a residual");  // no gate: 1
     TT_CHECK(ldr % 8 == 0 && gate_ld % 4 == 0 && (((uintptr_t)residual | (uintptr_t)gate) & 15) == 0,
              "gemm2: residual/gate misaligned");
   }

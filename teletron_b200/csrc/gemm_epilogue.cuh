@@ -111,8 +111,11 @@ __device__ __forceinline__ void epilogue_vec(const GemmParams& p, float (&v)[8],
     }
     uint4 rv = *reinterpret_cast<const uint4*>(p.residual + (long long)row * p.ldr + col);
     const uint32_t* ru = reinterpret_cast<const uint32_t*>(&rv);
-    float4 g0 = *reinterpret_cast<const float4*>(gate_row + col);
-    float4 g1 = *reinterpret_cast<const float4*>(gate_row + col + 4);
+    float4 g0 = make_float4(1.f, 1.f, 1.f, 1.f), g1 = g0;
+    if (gate_row) {
+      g0 = *reinterpret_cast<const float4*>(gate_row + col);
+      g1 = *reinterpret_cast<const float4*>(gate_row + col + 4);
+    }
     const float gg[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -160,7 +163,7 @@ template <int BN>
 __device__ __forceinline__ void epilogue_tile(const GemmParams& p, uint32_t acc, int eg, int row, bool row_ok,
                                               bf16* c_row, int n0) {
   const float* gate_row = nullptr;
-  if (p.epi == EPI_GATE_RES && row_ok)
+  if (p.epi == EPI_GATE_RES && p.gate && row_ok)
     gate_row = p.gate + (long long)(row / p.rows_per_gate) * p.gate_ld;
 #pragma unroll 1
   for (int c = eg * (BN / 64); c < (eg + 1) * (BN / 64); ++c) {

@@ -149,7 +149,7 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
       }
 #pragma unroll
       for (int j = 0; j < 8; ++j) v[j] *= p.alpha;
-      const float* gate_row = p.epi == EPI_GATE_RES ? p.gate + (long long)(row / p.rows_per_gate) * p.gate_ld : nullptr;
+      const float* gate_row = p.epi == EPI_GATE_RES && p.gate ? p.gate + (long long)(row / p.rows_per_gate) * p.gate_ld : nullptr;
       epilogue_vec(p, v, row, col, reinterpret_cast<bf16*>(p.C) + (long long)row * p.ldc, gate_row);
     }
   } else {

@@ -34,7 +34,7 @@ namespace {
 enum Par : int { P_MOD, P_QKV_W, P_QKV_B, P_NQ, P_NK, P_O_W, P_O_B, P_N3_W, P_N3_B, P_CQ_W, P_CQ_B, P_KV_W, P_KV_B, P_CNQ,
                  P_CNK, P_CO_W, P_CO_B, P_F1_W, P_F1_B, P_F2_W, P_F2_B };
 
-// small fp32 operands of the block: e [B][6][C] = modulation + t_mod, then six rows [C] of norm weights and one of ones
+// small fp32 operands of the block: e [B][6][C] = modulation + t_mod, then six rows [C] of norm weights
 struct PrepParams {
   const bf16* mod;
   const float* t_mod;
@@ -45,9 +45,9 @@ struct PrepParams {
 __global__ void __launch_bounds__(256) wan_prep_kernel(const PrepParams p) {
   const int row = blockIdx.y, c = blockIdx.x * 256 + threadIdx.x;
   if (c >= p.C) return;
-  float v = 1.f;
+  float v;
   if (row < 6 * p.B) v = __bfloat162float(p.mod[(row % 6) * p.C + c]) + p.t_mod[(long long)row * p.C + c];
-  else if (row < 6 * p.B + 6) v = __bfloat162float(p.rows[row - 6 * p.B][c]);
+  else v = __bfloat162float(p.rows[row - 6 * p.B][c]);
   p.out[(long long)row * p.C + c] = v;
 }
 
@@ -69,7 +69,7 @@ Work carve(uint8_t* base, int B, int S, int Lc, int C, int H, int F) {
   Carver c{base, 0};
   const long long R = (long long)B * S, Rc = (long long)B * Lc, Rk = R > Rc ? R : Rc;
   Work w;
-  w.small = (float*)c.take((6ll * B + 7) * C * 4);
+  w.small = (float*)c.take((6ll * B + 6) * C * 4);
   w.lse = (float*)c.take((long long)B * H * S * 4);
   w.h = (bf16*)c.take(R * C * 2);
   w.q = (bf16*)c.take(R * C * 2);
@@ -99,7 +99,7 @@ TT_API int tt_wan_block_fwd(const void* x, long long ldx, void* out, const void*
                             int freq_rows, const long long* params, int B, int S, int Lc, int C, int H, int F, float eps,
                             int pair, void* workspace, unsigned* status, cudaStream_t stream) {
   TT_CHECK(B > 0 && S > 0 && Lc > 0 && C > 0 && H > 0 && C == H * 128 && F > 0 && F % 8 == 0, "wan_block: bad shape");
-  TT_CHECK(6ll * B + 7 < 65536 && (long long)B * S < (1ll << 31) && (long long)B * Lc < (1ll << 31), "wan_block: too many rows");
+  TT_CHECK(6ll * B + 6 < 65536 && (long long)B * S < (1ll << 31) && (long long)B * Lc < (1ll << 31), "wan_block: too many rows");
   const Work w = carve((uint8_t*)workspace, B, S, Lc, C, H, F);
   const int R = B * S, Rc = B * Lc, D = 128;
   const float scale = (float)(1.0 / sqrt((double)D));
@@ -108,7 +108,7 @@ TT_API int tt_wan_block_fwd(const void* x, long long ldx, void* out, const void*
   pp.mod = par(P_MOD); pp.t_mod = t_mod; pp.out = w.small; pp.B = B; pp.C = C;
   const int rows6[6] = {P_NQ, P_NK, P_N3_W, P_N3_B, P_CNQ, P_CNK};
   for (int i = 0; i < 6; ++i) pp.rows[i] = par(rows6[i]);
-  wan_prep_kernel<<<dim3((C + 255) / 256, 6 * B + 7), 256, 0, stream>>>(pp);
+  wan_prep_kernel<<<dim3((C + 255) / 256, 6 * B + 6), 256, 0, stream>>>(pp);
   TT_LAUNCH_CHECK();
   auto ev = [&](int i) { return w.small + (long long)i * C; };         // row i of sample 0; samples are 6 * C apart
   auto sm = [&](int i) { return w.small + (6ll * B + i) * C; };
@@ -146,7 +146,7 @@ TT_API int tt_wan_block_fwd(const void* x, long long ldx, void* out, const void*
   TT_RUN(tt_rmsrope_fwd(w.kv, 2 * C, w.k, C, sm(5), nullptr, 1, nullptr, Rc, C, D, 0, eps, stream));
   TT_RUN(tt_attn_fwd(w.q, C, sc, w.k, C, (long long)Lc * C, w.kv + C, 2 * C, lc2, w.a, C, sc, w.lse, nullptr, B, H, S, Lc, D,
                      scale, status, stream));
-  TT_RUN(gemm(w.a, C, P_CO_W, w.x2, R, C, C, GATE_RES, w.x1, C, sm(6), C, R));
+  TT_RUN(gemm(w.a, C, P_CO_W, w.x2, R, C, C, GATE_RES, w.x1, C, nullptr, 0, R));
   // feed-forward
   TT_RUN(tt_adaln_fwd(w.x2, C, w.h, C, ev(4), ev(3), e_ld, 1, R, C, S, eps, nullptr, nullptr, stream));
   TT_RUN(gemm(w.h, C, P_F1_W, w.mid, R, F, C, GELU, nullptr, 0, nullptr, 0, 1));

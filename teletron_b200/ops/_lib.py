@@ -118,6 +118,21 @@ def check_status(device: torch.device | None = None) -> None:
                            "results of this step are invalid")
 
 
+def main_grad_of(p):
+    """The fp32 gradient buffer of a parameter (set by ``parallel.ddp.ParamBuffer``) when kernels may add to it."""
+    mg = getattr(p, "main_grad", None)
+    return mg if mg is not None and mg.dtype == torch.float32 and mg.is_contiguous() else None
+
+
+def grad_written(p) -> None:
+    """A kernel has added this parameter's gradient to its buffer: lets the optimizer start the reduction of the
+    parameter's bucket (parallel/ddp.py)."""
+    p.grad_written = True
+    ready = getattr(p, "grad_ready", None)
+    if ready is not None:
+        ready()
+
+
 def launch_count() -> int:
     """Kernels launched by the native library in this process so far."""
     return int(lib().tt_launch_count()) if lib_file().exists() else 0

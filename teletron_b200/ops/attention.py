@@ -148,6 +148,7 @@ class _SelfAttnCore(torch.autograd.Function):
         o, lse = attention_fwd(q4, k4, v4)
         ctx.save_for_backward(qkv, wqf, wkf, freqs, rq, rk, q, k, o, lse)
         ctx.meta = (batch, S, H, D, wq.dtype)
+        ctx.owners = (wq if ctx.needs_input_grad[1] else None, wk if ctx.needs_input_grad[2] else None)
         return o.view(batch * S, C)
 
     @staticmethod
@@ -166,10 +167,12 @@ class _SelfAttnCore(torch.autograd.Function):
         v4 = qkv[:, 2 * C:3 * C].unflatten(1, (H, D)).unflatten(0, (batch, S))
         attention_bwd(q.view(batch, S, H, D), k.view(batch, S, H, D), v4, o, lse, do.view(batch, S, H, D),
                       out=(dqn, dkn, dv_view))
-        _, dwq = rmsrope_bwd_raw(dqn.view(batch * S, C), qkv[:, 0:C], wqf, freqs, rq, D, False, out=dqkv[:, 0:C])
+        _, dwq = rmsrope_bwd_raw(dqn.view(batch * S, C), qkv[:, 0:C], wqf, freqs, rq, D, False, out=dqkv[:, 0:C],
+                                 owner=ctx.owners[0])
         _, dwk = rmsrope_bwd_raw(dkn.view(batch * S, C), qkv[:, C:2 * C], wkf, freqs, rk, D, False,
-                                 out=dqkv[:, C:2 * C])
-        return dqkv, dwq.to(wdtype), dwk.to(wdtype), None, None, None, None, None, None
+                                 out=dqkv[:, C:2 * C], owner=ctx.owners[1])
+        dwq, dwk = (None if g is None else g.to(wdtype) for g in (dwq, dwk))
+        return dqkv, dwq, dwk, None, None, None, None, None, None
 
 
 def self_attention_core(qkv, wq, wk, freqs, batch, S, H, D, eps=1e-6):

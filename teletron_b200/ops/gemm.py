@@ -52,7 +52,7 @@ def gemm_ref(a, b, *, a_mn=False, b_mn=False, bias=None, epi=EPI_NONE, residual=
         acc = torch.nn.functional.silu(acc)
     elif epi == EPI_GATE_RES:
         aux = acc.to(torch.bfloat16) if want_aux else None
-        g = gate.float().repeat_interleave(rows_per_gate, dim=0)[: acc.shape[0]]
+        g = 1.0 if gate is None else gate.float().repeat_interleave(rows_per_gate, dim=0)[: acc.shape[0]]
         acc = residual.float() + g * acc
     elif epi == EPI_ACCUM:
         acc = out.float() + acc
@@ -71,7 +71,7 @@ def gemm(a, b, *, a_mn=False, b_mn=False, bias=None, epi=EPI_NONE, residual=None
     a: [M,K] (or [K,M] when a_mn)   b: [N,K] (or [K,N] when b_mn); both bf16 with a
     contiguous last dim.  ``epi``: EPI_GELU / EPI_SILU (optionally returning the
     pre-activation as aux), EPI_GATE_RES (``residual + gate[row // rows_per_gate] * acc``,
-    gate fp32), EPI_ACCUM (``out += acc``).
+    gate fp32, None = 1), EPI_ACCUM (``out += acc``).
     """
     if not a.is_cuda:
         return gemm_ref(a, b, a_mn=a_mn, b_mn=b_mn, bias=bias, epi=epi, residual=residual, gate=gate,
@@ -101,8 +101,8 @@ def gemm(a, b, *, a_mn=False, b_mn=False, bias=None, epi=EPI_NONE, residual=None
     if bias is not None:
         assert bias.dtype == torch.bfloat16 and bias.is_contiguous() and bias.numel() == N
     if epi == EPI_GATE_RES:
-        assert residual.dtype == torch.bfloat16 and gate.dtype == torch.float32
-        assert residual.shape == (M, N) and residual.stride(1) == 1 and gate.stride(-1) == 1
+        assert residual.dtype == torch.bfloat16 and residual.shape == (M, N) and residual.stride(1) == 1
+        assert gate is None or (gate.dtype == torch.float32 and gate.stride(-1) == 1)
     L = _lib.lib()
     if _PAIR and max_ctas == 0 and M >= 256 and N >= 256:
         rc = L.tt_gemm2_bf16(

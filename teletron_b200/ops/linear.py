@@ -19,6 +19,7 @@ import torch
 import torch.nn.functional as F
 
 from . import _lib
+from ._lib import grad_written, main_grad_of
 from .gemm import EPI_ACCUM, EPI_GATE_RES, EPI_GELU, EPI_NONE, EPI_SILU, gemm
 
 _ACT = {None: EPI_NONE, "gelu": EPI_GELU, "silu": EPI_SILU}
@@ -26,16 +27,17 @@ _ACT = {None: EPI_NONE, "gelu": EPI_GELU, "silu": EPI_SILU}
 _COLSUM_CHUNKS = 296
 
 
-def colsum(x: torch.Tensor, out_dtype=torch.float32) -> torch.Tensor:
-    """Column sums of a bf16 [rows, C] matrix (bias gradients)."""
+def colsum(x: torch.Tensor, out_dtype=torch.float32, add_to=None) -> torch.Tensor:
+    """Column sums of a bf16 [rows, C] matrix (bias gradients), or added to the fp32 vector ``add_to``."""
     if not x.is_cuda:
-        return x.float().sum(0).to(out_dtype)
+        s = x.float().sum(0)
+        return s.to(out_dtype) if add_to is None else add_to.add_(s)
     rows, C = x.shape
     chunks = max(1, min(rows, _COLSUM_CHUNKS))
     partial = torch.empty((chunks, C), dtype=torch.float32, device=x.device)
-    out = torch.empty(C, dtype=out_dtype, device=x.device)
+    out = torch.empty(C, dtype=out_dtype, device=x.device) if add_to is None else add_to
     rc = _lib.lib().tt_colsum(_lib.ptr(x), _lib.c_ll(x.stride(0)), _lib.ptr(partial), _lib.c_int(chunks),
-                              _lib.ptr(out), _lib.c_int(int(out_dtype == torch.float32)), _lib.c_int(0),
+                              _lib.ptr(out), _lib.c_int(int(out.dtype == torch.float32)), _lib.c_int(int(add_to is not None)),
                               _lib.c_int(rows), _lib.c_int(C), _lib.stream())
     _lib.check(rc, "tt_colsum")
     return out
@@ -63,16 +65,20 @@ def _weight_grad(dy, x, w, owner=None):
     mg = getattr(w, "main_grad", None)
     if mg is not None:
         gemm(dy, x, a_mn=True, b_mn=True, out=mg, epi=EPI_ACCUM)
-        w.grad_written = True
-        ready = getattr(w, "grad_ready", None)
-        if ready is not None:      # lets the optimizer start this parameter's bucket reduction (parallel/ddp.py)
-            ready()
+        grad_written(w)
         return None
     return gemm(dy, x, a_mn=True, b_mn=True, out_dtype=w.dtype)
 
 
 def _bias_grad(dy, b):
+    """Column sums of dy: added to the parameter's fp32 gradient buffer when it has one (returns None: no bf16 copy,
+    no accumulation in bf16 over micro-batches, no fold afterwards), else a gradient of the bias' type."""
     if b is None:
+        return None
+    mg = main_grad_of(b)
+    if mg is not None and dy.is_cuda and mg.numel() == dy.shape[1]:
+        colsum(dy, add_to=mg.view(-1))
+        grad_written(b)
         return None
     return colsum(dy, out_dtype=torch.float32).to(b.dtype)
 
@@ -122,12 +128,7 @@ class _LinearResidual(torch.autograd.Function):
     def forward(ctx, x, w, b, res, gate, rows_per_gate):
         rows = x.shape[0]
         has_gate = gate is not None
-        if has_gate:
-            g = gate
-            rpg = rows_per_gate
-        else:
-            g = torch.ones((1, w.shape[0]), dtype=torch.float32, device=x.device)
-            rpg = rows
+        g, rpg = (gate, rows_per_gate) if has_gate else (None, rows)
         need_z = has_gate and ctx.needs_input_grad[4]
         if need_z:
             y, z = gemm(x, w, bias=b, epi=EPI_GATE_RES, residual=res, gate=g, rows_per_gate=rpg, want_aux=True)
@@ -221,17 +222,14 @@ class _RowLinear(torch.autograd.Function):
                                             _lib.c_int(B * K), _lib.c_int(0), _lib.stream()), "tt_colsum_partials")
         if ctx.needs_input_grad[1]:
             owner = ctx.w_param
-            mg = getattr(owner, "main_grad", None)
-            into_main = mg is not None and mg.dtype == torch.float32 and mg.is_contiguous() and mg.data_ptr() % 16 == 0
+            mg = main_grad_of(owner)
+            into_main = mg is not None and mg.data_ptr() % 16 == 0
             dw = mg if into_main else torch.empty((N, K), dtype=torch.bfloat16, device=x.device)
             _lib.check(L.tt_rowlin_wgrad(_lib.ptr(dy), _lib.ptr(x), _lib.ptr(dw), _lib.c_int(int(into_main)), *dims,
                                          _lib.stream()), "tt_rowlin_wgrad")
             if into_main:
                 dw = None
-                owner.grad_written = True
-                ready = getattr(owner, "grad_ready", None)
-                if ready is not None:
-                    ready()
+                grad_written(owner)
         if ctx.bias_dtype is not None and ctx.needs_input_grad[2]:
             db = dy.sum(0).to(ctx.bias_dtype)
         return dx, dw, db

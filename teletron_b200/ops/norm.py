@@ -40,10 +40,12 @@ def adaln_ref(x, scale, shift, rows_per_batch, eps=1e-6, plus_one=True):
 
 class _AdaLN(torch.autograd.Function):
     """``with_res``: also return x itself as a second output (an alias) for the residual connection, so that
-    the residual's gradient arrives here and is added inside the backward kernel (no separate add kernel)."""
+    the residual's gradient arrives here and is added inside the backward kernel (no separate add kernel).
+    ``owners``: the (weight, bias) parameters behind scale and shift when their gradients go straight into the
+    parameters' fp32 buffers."""
 
     @staticmethod
-    def forward(ctx, x, scale, shift, rows_per_batch, eps, plus_one, with_res=False):
+    def forward(ctx, x, scale, shift, rows_per_batch, eps, plus_one, with_res=False, owners=None):
         rows, C = x.shape
         assert x.dtype == torch.bfloat16 and x.stride(1) == 1
         for m in (scale, shift):
@@ -64,6 +66,7 @@ class _AdaLN(torch.autograd.Function):
         _lib.check(rc, "tt_adaln_fwd")
         ctx.save_for_backward(x, mean, rstd, scale)
         ctx.meta = (rows_per_batch, plus_one, batch, mod_ld, shift is not None)
+        ctx.owners = owners
         if with_res:
             return y, x.view_as(x)
         return y
@@ -75,28 +78,37 @@ class _AdaLN(torch.autograd.Function):
         rows, C = x.shape
         assert rows == batch * rows_per_batch, "adaln backward needs rows == batch * rows_per_batch"
         if dy is None:  # only the residual alias was used
-            return dres, None, None, None, None, None, None
+            return dres, None, None, None, None, None, None, None
         if dy.stride(1) != 1:
             dy = dy.contiguous()
         if dres is not None and (dres.dtype != torch.bfloat16 or dres.stride(1) != 1):
             dres = dres.to(torch.bfloat16).contiguous()
         dx = torch.empty((rows, C), dtype=torch.bfloat16, device=x.device)
-        want_mod = (scale is not None and ctx.needs_input_grad[1]) or (has_shift and ctx.needs_input_grad[2])
+        owners = ctx.owners
+        want_mod = (owners is not None or (scale is not None and ctx.needs_input_grad[1])
+                    or (has_shift and ctx.needs_input_grad[2]))
         chunks = _chunks(rows_per_batch, batch)
         partial = dmul = dadd = None
         if want_mod:
             partial = torch.empty((batch, chunks, 2, C), dtype=torch.float32, device=x.device)
-            dmul = torch.empty((batch, C), dtype=torch.float32, device=x.device) if scale is not None else None
-            dadd = torch.empty((batch, C), dtype=torch.float32, device=x.device) if has_shift else None
+            if owners is not None:
+                dmul, dadd = (_lib.main_grad_of(p) for p in owners)
+            else:
+                dmul = torch.empty((batch, C), dtype=torch.float32, device=x.device) if scale is not None else None
+                dadd = torch.empty((batch, C), dtype=torch.float32, device=x.device) if has_shift else None
         rc = _lib.lib().tt_adaln_bwd(
             _lib.ptr(dy), _lib.c_ll(dy.stride(0)), _lib.ptr(x), _lib.c_ll(x.stride(0)), _lib.ptr(mean),
             _lib.ptr(rstd), _lib.ptr(scale), _lib.c_ll(mod_ld), _lib.c_int(int(plus_one)), _lib.ptr(dx),
             _lib.c_ll(C), _lib.ptr(dres), _lib.c_ll(dres.stride(0) if dres is not None else 0), _lib.ptr(partial),
             _lib.c_int(chunks),
-            _lib.ptr(dmul), _lib.ptr(dadd), _lib.c_int(0), _lib.c_int(batch), _lib.c_int(rows_per_batch),
+            _lib.ptr(dmul), _lib.ptr(dadd), _lib.c_int(int(owners is not None)), _lib.c_int(batch), _lib.c_int(rows_per_batch),
             _lib.c_int(C), _lib.stream())
         _lib.check(rc, "tt_adaln_bwd")
-        return dx, dmul, dadd, None, None, None, None
+        if owners is not None:
+            for p in owners:
+                _lib.grad_written(p)
+            dmul = dadd = None
+        return dx, dmul, dadd, None, None, None, None, None
 
 
 def adaln(x, scale, shift, rows_per_batch, eps=1e-6, plus_one=True):
@@ -117,6 +129,12 @@ def adaln_res(x, scale, shift, rows_per_batch, eps=1e-6, plus_one=True):
 def layernorm_affine(x, weight, bias, eps=1e-6, with_res=False):
     """nn.LayerNorm with affine parameters (Wan ``norm3``) through the AdaLN kernel."""
     rows = x.shape[0]
+    if (x.is_cuda and weight is not None and bias is not None and torch.is_grad_enabled() and weight.requires_grad
+            and bias.requires_grad and _lib.main_grad_of(weight) is not None and _lib.main_grad_of(bias) is not None):
+        # the parameters stay inputs of the node, so that autograd runs their hooks
+        w, b = weight.float().unsqueeze(0), bias.float().unsqueeze(0)
+        out = _AdaLN.apply(x, w, b, rows, eps, False, with_res, (weight, bias))
+        return out
     w = weight.float().unsqueeze(0) if weight is not None else None
     b = bias.float().unsqueeze(0) if bias is not None else None
     if with_res:
@@ -180,19 +198,21 @@ class _RmsRope(torch.autograd.Function):
         y, rstd = rmsrope_fwd_raw(x, wf, freqs, D, per_head, eps)
         ctx.save_for_backward(x, wf, freqs, rstd)
         ctx.meta = (D, per_head, weight.dtype if weight is not None else None)
+        ctx.owner = weight if weight is not None and ctx.needs_input_grad[1] else None
         return y
 
     @staticmethod
     def backward(ctx, dy):
         x, wf, freqs, rstd = ctx.saved_tensors
         D, per_head, wdtype = ctx.meta
-        dx, dw = rmsrope_bwd_raw(dy, x, wf, freqs, rstd, D, per_head)
+        dx, dw = rmsrope_bwd_raw(dy, x, wf, freqs, rstd, D, per_head, owner=ctx.owner)
         return dx, (dw.to(wdtype) if dw is not None else None), None, None, None, None
 
 
-def rmsrope_bwd_raw(dy, x, wf, freqs, rstd, D, per_head=False, out=None):
+def rmsrope_bwd_raw(dy, x, wf, freqs, rstd, D, per_head=False, out=None, owner=None):
     """Backward of rope(rmsnorm(x) * w) from the saved input and rstd: returns (dx bf16, dw fp32 or None).
-    ``out``: optional [rows, C] view (any row stride) that receives dx."""
+    ``out``: optional [rows, C] view (any row stride) that receives dx.  ``owner``: the weight parameter; a full-row
+    weight gradient is added to its fp32 buffer when it has one (dw is None then)."""
     rows, C = x.shape
     if dy.stride(1) != 1:
         dy = dy.contiguous()
@@ -211,10 +231,14 @@ def rmsrope_bwd_raw(dy, x, wf, freqs, rstd, D, per_head=False, out=None):
     _lib.check(rc, "tt_rmsrope_bwd")
     dw = None
     if wf is not None:
-        dwf = torch.empty((1, C), dtype=torch.float32, device=x.device)
+        mg = None if owner is None or per_head else _lib.main_grad_of(owner)
+        dwf = torch.empty((1, C), dtype=torch.float32, device=x.device) if mg is None else mg
         rc = L.tt_colsum_partials(_lib.ptr(partial), _lib.ptr(dwf), _lib.c_int(1), _lib.c_int(ctas),
-                                  _lib.c_int(C), _lib.c_int(0), _lib.stream())
+                                  _lib.c_int(C), _lib.c_int(int(mg is not None)), _lib.stream())
         _lib.check(rc, "tt_colsum_partials")
+        if mg is not None:
+            _lib.grad_written(owner)
+            return dx, None
         dw = dwf.view(C // D, D).sum(0) if per_head else dwf.view(C)
     return dx, dw
 
