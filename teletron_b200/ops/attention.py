@@ -34,8 +34,8 @@ def _check_layout(t: torch.Tensor, name: str):
         f"{name}: expected [B,S,H,D] with dense (H,D), got strides {t.stride()}")
 
 
-def attention_fwd(q, k, v, scale=None, kv_lens=None):
-    """Returns (o [B,Sq,H,D] bf16 contiguous, lse [B,H,Sq] fp32)."""
+def attention_fwd(q, k, v, scale=None, kv_lens=None, out=None):
+    """Returns (o [B,Sq,H,D] bf16 contiguous, or written into the view ``out`` with dense (H, D), lse [B,H,Sq] fp32)."""
     B, Sq, H, D = q.shape
     Skv = k.shape[1]
     scale = scale if scale is not None else 1.0 / math.sqrt(D)
@@ -44,7 +44,9 @@ def attention_fwd(q, k, v, scale=None, kv_lens=None):
     for t, n in ((q, "q"), (k, "k"), (v, "v")):
         _check_layout(t, n)
         assert t.dtype == torch.bfloat16
-    o = torch.empty((B, Sq, H, D), dtype=torch.bfloat16, device=q.device)
+    o = torch.empty((B, Sq, H, D), dtype=torch.bfloat16, device=q.device) if out is None else out
+    _check_layout(o, "out")
+    assert o.shape == q.shape and o.dtype == torch.bfloat16
     lse = torch.empty((B, H, Sq), dtype=torch.float32, device=q.device)
     if kv_lens is not None:
         kv_lens = kv_lens.to(device=q.device, dtype=torch.int32).contiguous()

@@ -172,14 +172,15 @@ def rmsnorm_rope_ref(x, weight, freqs, D, per_head=False, eps=1e-6):
     return xf.to(x.dtype)
 
 
-def rmsrope_fwd_raw(x, wf, freqs, D, per_head=False, eps=1e-6):
+def rmsrope_fwd_raw(x, wf, freqs, D, per_head=False, eps=1e-6, out=None):
     """rope(rmsnorm(x) * wf) without autograd: returns (y bf16 [rows, C], rstd fp32 or None). ``x`` may be a
-    column slice of a wider tensor (row stride > C)."""
+    column slice of a wider tensor (row stride > C); ``out``: optional dense [rows, C] that receives y."""
     rows, C = x.shape
     assert x.dtype == torch.bfloat16 and x.stride(1) == 1
     if freqs is not None:
         assert freqs.dtype == torch.float32 and freqs.is_contiguous() and freqs.shape[1:] == (D // 2, 2)
-    y = torch.empty((rows, C), dtype=torch.bfloat16, device=x.device)
+    y = torch.empty((rows, C), dtype=torch.bfloat16, device=x.device) if out is None else out
+    assert y.shape == (rows, C) and y.dtype == torch.bfloat16 and y.is_contiguous()
     rstd = None
     if wf is not None:
         rstd = torch.empty(rows * (C // D if per_head else 1), dtype=torch.float32, device=x.device)
