@@ -10,6 +10,7 @@ from __future__ import annotations
 import torch
 import torch.nn as nn
 
+from ... import ops
 from ...ops import conv as C
 from . import wan_vae as V
 
@@ -113,7 +114,23 @@ class Run:
         return self.norm_conv(r[3], r[6], h, res=skip)
 
     def attention(self, m, x):
-        return C.from_planar(m(C.to_planar(x).unsqueeze(0)).squeeze(0))
+        """Single-head attention over the pixels of each frame (heads of up to 384 channels)."""
+        t, chunks, h, w, e = x.shape
+        n, c = h * w, chunks * e
+        if x.dtype != torch.bfloat16 or n > 32768:
+            return C.from_planar(m(C.to_planar(x).unsqueeze(0)).squeeze(0))
+        y = C.chan_norm(x, m.norm.gamma.detach().reshape(-1), torch.empty_like(x), act=False)
+        qkv = self.conv(m.to_qkv, C.CONV_POINT, y, t, (h, w))
+        padded = -(-n // 8) * 8                            # keys in whole vectors; the softmax stops at n
+        rows = qkv.new_zeros((t, padded, 3 * c))
+        rows[:, :n].unflatten(1, (h, w)).unflatten(3, (3 * chunks, e)).copy_(qkv.permute(0, 2, 3, 1, 4))
+        out = torch.empty((t, n, c), dtype=x.dtype, device=x.device)
+        for f in range(t):
+            q, k, v = rows[f, :n, :c], rows[f, :, c:2 * c], rows[f, :, 2 * c:]
+            scores = ops.gemm(q, k, out_dtype=torch.float32, alpha=c ** -0.5)
+            ops.gemm(C.softmax_split(scores, n), torch.cat([v, v]), b_mn=True, out=out[f])
+        o = C.from_planar(out.view(t, h, w, c).permute(3, 0, 1, 2))
+        return self.conv(m.proj, C.CONV_POINT, o, t, (h, w), res=x)
 
     def down(self, m, x):
         st = V._STREAM

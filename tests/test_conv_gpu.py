@@ -78,6 +78,37 @@ def test_chan_norm(dtype, c):
     _close(y, ref, dtype)
 
 
+@pytest.mark.parametrize("rows,n", [(3, 1), (5, 8), (64, 1023), (7, 6240), (2, 1032)])
+def test_softmax_split(rows, n):
+    torch.manual_seed(4)
+    padded = -(-n // 8) * 8
+    s = torch.randn(rows, padded, device="cuda") * 4
+    s[:, n:] = float("nan")                                   # not read
+    s[0, 0] = -float("inf") if n > 1 else 0.0
+    p = C.softmax_split(s, n)
+    ref = torch.softmax(s[:, :n].double(), dim=1)
+    got = p[:, :padded].double() + p[:, padded:].double()
+    assert (got[:, n:] == 0).all()
+    # two bf16 parts: 2^-17 of the value
+    assert ((got[:, :n] - ref).norm() / ref.norm()).item() < 2 ** -16
+
+
+@pytest.mark.parametrize("t,h,w", [(2, 5, 7), (1, 30, 53), (1, 2, 2)])
+def test_frame_attention(t, h, w):
+    """Against fp64; the error may not exceed the library path's."""
+    torch.manual_seed(5)
+    m = wan_vae.AttentionBlock(384)
+    torch.nn.init.normal_(m.proj.weight, std=0.05)
+    m = m.to("cuda", torch.bfloat16).requires_grad_(False)
+    x = _rand(384, t, h, w, dtype=torch.bfloat16)
+    out = C.to_planar(wan_vae_native.Run().attention(m, C.from_planar(x)))
+    old = m(x[None])[0]
+    ref = m.double()(x.double()[None])[0]
+    e_new, e_old = (((a.double() - ref).norm() / ref.norm()).item() for a in (out, old))
+    assert e_new <= e_old * 1.05 + 1e-5, (e_new, e_old)
+    _lib.check_status()
+
+
 def _vae(dtype, dim):
     torch.manual_seed(3)
     vae = WanVideoVAE(dim=dim)
