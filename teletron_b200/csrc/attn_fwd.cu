@@ -69,6 +69,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   const int h = blockIdx.y;
   const int b = blockIdx.z;
   int kv_len = p.Skv;
+  chain_release();
+  if (p.kv_lens) chain_wait();
   if (p.kv_lens) kv_len = min(max(p.kv_lens[b], 1), p.Skv);
   const int n_tiles = (kv_len + TILE - 1) / TILE;
 
@@ -99,6 +101,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  chain_wait();
 
   if (warp == 0) {
     // ---------------------------------------------------------------- producer
@@ -344,7 +347,7 @@ static int attn_fwd_impl(const void* q, long long ldq, long long q_bs, const voi
     attr_done = true;
   }
   dim3 grid((Sq + 2 * TILE - 1) / (2 * TILE), H, B);
-  attn_fwd_kernel<<<grid, NTHREADS, SMEM_BYTES, stream>>>(tmQ, tmK, tmV, p);
+  TT_CUDA(tt_launch(attn_fwd_kernel, grid, dim3(NTHREADS), SMEM_BYTES, stream, 1, tmQ, tmK, tmV, p));
   TT_LAUNCH_CHECK();
   return 0;
 }

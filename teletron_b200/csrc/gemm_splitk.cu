@@ -42,6 +42,7 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   const int num_kb = (p.K + BK - 1) / BK;
   const int kb0 = (int)((long long)num_kb * rank / split), kb1 = (int)((long long)num_kb * (rank + 1) / split);
 
+  chain_release();
   if (threadIdx.x == 0) {
     for (int s = 0; s < SK_STAGES; ++s) {
       mbar_init(&full[s], 1);
@@ -63,6 +64,7 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  chain_wait();
   float* park = reinterpret_cast<float*>(smem);
 
   if (warp == 0) {
@@ -165,19 +167,7 @@ int launch_splitk(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmPara
   auto kern = gemm_splitk_kernel<A_MN, B_MN>;
   TT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SK_SMEM));
   const int tiles = ((p.M + BM - 1) / BM) * ((p.N + SK_BN - 1) / SK_BN);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(tiles * split, 1, 1);
-  cfg.blockDim = dim3(320, 1, 1);
-  cfg.dynamicSmemBytes = SK_SMEM;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = split;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  TT_CUDA(cudaLaunchKernelEx(&cfg, kern, tmA, tmB, p, split));
+  TT_CUDA(tt_launch(kern, dim3(tiles * split), dim3(320), SK_SMEM, stream, split, tmA, tmB, p, split));
   TT_LAUNCH_CHECK();
   return 0;
 }

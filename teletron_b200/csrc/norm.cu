@@ -160,6 +160,8 @@ adaln_fwd_warp_kernel(const bf16* __restrict__ x, long long ldx, bf16* __restric
   const float invC = 1.f / (float)C;
   const int first_row = blockIdx.x * (NT / 32);
   const int cached_b = first_row < rows ? first_row / rows_per_batch : -1;
+  chain_release();
+  chain_wait();
   if (cached_b >= 0) {
     for (int i = threadIdx.x; i < C; i += NT) {
       const float mv = mul ? mul[(long long)cached_b * mod_ld + i] : (plus_one ? 0.f : 1.f);
@@ -520,8 +522,8 @@ TT_API int tt_adaln_fwd(const void* x, long long ldx, void* y, long long ldy, co
     const int want = (rows + NT / 32 - 1) / (NT / 32);
     const int wgrid = want < 148 * 8 ? want : 148 * 8;
 #define TT_ADALN_WARP(NVV)                                                                                   \
-  adaln_fwd_warp_kernel<NVV><<<wgrid, NT, 0, stream>>>((const bf16*)x, ldx, (bf16*)y, ldy, mul, add, mod_ld, \
-                                                       plus_one, rows, rows_per_batch, eps, mean_out, rstd_out)
+  TT_CUDA(tt_launch(adaln_fwd_warp_kernel<NVV>, dim3(wgrid), dim3(NT), 0, stream, 1, (const bf16*)x, ldx, (bf16*)y, ldy, mul, add, \
+                    mod_ld, plus_one, rows, rows_per_batch, eps, mean_out, rstd_out))
     switch (C / 256) {
       case 1: TT_ADALN_WARP(1); break;
       case 2: TT_ADALN_WARP(2); break;
@@ -616,6 +618,8 @@ rmsrope_fwd_warp_kernel(const bf16* __restrict__ in, long long ldi, bf16* __rest
   __shared__ __align__(16) float w_s[C];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int vec_per_head = D >> 3;
+  chain_release();
+  chain_wait();
   for (int i = threadIdx.x; i < C; i += NT) w_s[i] = w ? w[PER_HEAD ? i % D : i] : 1.f;
   __syncthreads();
   for (int row = blockIdx.x * (NT / 32) + warp; row < rows; row += gridDim.x * (NT / 32)) {
@@ -912,8 +916,8 @@ static int rmsrope_fwd_impl(const void* x, long long ldx, void* y, long long ldy
 #define TT_RMS_FWD_WARP(NVV)                                                                                              \
   do {                                                                                                                    \
     auto kern = per_head ? rmsrope_fwd_warp_kernel<NVV, true> : rmsrope_fwd_warp_kernel<NVV, false>;                      \
-    kern<<<wgrid, NT, 0, stream>>>((const bf16*)x, ldx, (bf16*)y, ldy, w, (const float2*)freqs, freq_rows, rstd, rows, D, \
-                                   eps, sc, ssq, ssq_n, ssq_ld);                                                          \
+    TT_CUDA(tt_launch(kern, dim3(wgrid), dim3(NT), 0, stream, 1, (const bf16*)x, ldx, (bf16*)y, ldy, w,                   \
+                      (const float2*)freqs, freq_rows, rstd, rows, D, eps, sc, ssq, ssq_n, ssq_ld));                      \
   } while (0)
     switch (C / 256) {
       case 1: TT_RMS_FWD_WARP(1); break;

@@ -51,6 +51,45 @@ void tt_count_launch();
     TT_CUDA(cudaGetLastError());   \
   } while (0)
 
+// Launches inside a TTChain scope (one thread, one stream) overlap their start-up with the end of the launch before:
+// the kernel may be scheduled once every CTA of its predecessor has called tt::chain_release(), sets itself up, and
+// blocks in tt::chain_wait() until the predecessor has completed and its writes are visible.  Every kernel launched
+// through tt_launch calls chain_wait() before its first access to memory that another launch of the chain touches, so
+// the order of effects is that of the stream.  Kernels launched in the ordinary way before, between or after wait, and
+// are waited for, in full.
+bool& tt_chain_flag();  // thread-local
+struct TTChain {
+  bool old;
+  explicit TTChain(bool on) : old(tt_chain_flag()) { tt_chain_flag() = on; }
+  ~TTChain() { tt_chain_flag() = old; }
+};
+#ifdef __CUDACC__
+template <class... P, class... A>
+cudaError_t tt_launch(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int cluster, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  int n = 0;
+  if (cluster > 1) {
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = cluster;
+    attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
+    ++n;
+  }
+  if (tt_chain_flag()) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n].val.programmaticStreamSerializationAllowed = 1;
+    ++n;
+  }
+  cfg.attrs = attr;
+  cfg.numAttrs = n;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+#endif
+
 // Builds a tiled TMA descriptor for a row-major bf16/fp32 tensor of up to 4 dims.
 // dims[0] is the innermost (contiguous) extent; strides_bytes[i] is the stride of
 // dims[i+1]. Returns 0 on success.
@@ -111,6 +150,9 @@ __device__ __forceinline__ bf16* scatter_dst(const TTScatter& sc, int b, int tok
 __device__ __forceinline__ bool scatter_row(const TTScatter& sc, int row, int rows_total) {
   return sc.mode == 2 && row < rows_total && (sc.n_rows == 0 || row < sc.n_rows);
 }
+
+__device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));

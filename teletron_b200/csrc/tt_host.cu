@@ -16,6 +16,11 @@ void tt_set_error(const char* fmt, ...) {
   va_end(ap);
 }
 
+bool& tt_chain_flag() {
+  static thread_local bool on = false;
+  return on;
+}
+
 TT_API const char* tt_last_error() { return g_err; }
 
 static std::atomic<long long> g_launches{0};
