@@ -424,7 +424,7 @@ chan_norm_kernel(const uint4* __restrict__ x, uint4* __restrict__ y, const void*
   __syncthreads();
   if (!in) return;
   const float nrm = sqrtf((red[0][px] + red[1][px]) + (red[2][px] + red[3][px]));
-  const float inv = scale / fmaxf(nrm, 1e-12f);
+  const float inv = scale / (nrm < 1e-12f ? 1e-12f : nrm);  // a NaN stays one
 #pragma unroll
   for (int k = 0; k < NCH; ++k) {
     const int c = sl + 4 * k;

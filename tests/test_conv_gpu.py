@@ -76,6 +76,10 @@ def test_chan_norm(dtype, c):
     y = C.to_planar(C.chan_norm(xb, g, torch.empty_like(xb)))
     ref = F.silu(F.normalize(x.double(), dim=0) * c ** 0.5 * g.double().view(-1, 1, 1, 1))
     _close(y, ref, dtype)
+    x[3, 1, 2, 2] = float("nan")                              # spreads over its pixel, and no further
+    xb = C.from_planar(x)
+    bad = C.to_planar(C.chan_norm(xb, g, torch.empty_like(xb))).isnan()
+    assert bad[:, 1, 2, 2].all() and bad.sum() == c
 
 
 @pytest.mark.parametrize("rows,n", [(3, 1), (5, 8), (64, 1023), (7, 6240), (2, 1032)])
@@ -175,6 +179,12 @@ def test_route_to_the_modules():
         assert not wan_vae_native.usable(net, x)
     finally:
         torch.backends.cudnn.allow_tf32 = old
+    old = torch.backends.cudnn.conv.fp32_precision
+    try:
+        torch.backends.cudnn.conv.fp32_precision = "ieee"
+        assert not wan_vae_native.usable(net, x)
+    finally:
+        torch.backends.cudnn.conv.fp32_precision = old
     handle = net.conv1.register_forward_hook(lambda *a: None)
     assert not wan_vae_native.usable(net, x)
     handle.remove()
