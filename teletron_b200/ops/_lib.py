@@ -124,13 +124,30 @@ def main_grad_of(p):
     return mg if mg is not None and mg.dtype == torch.float32 and mg.is_contiguous() else None
 
 
+def main_grad_target(p):
+    """``main_grad_of(p)`` when the backward pass in progress may add p's gradient there and return None for it, else
+    None.  It may not when somebody is to see the gradient: ``autograd.grad`` hands it out, ``backward(inputs=...)`` may
+    leave p out, tensor hooks and post-accumulate hooks (other than the optimizer's) read it.  Autograd runs p's
+    AccumulateGrad once all uses of p in the pass are done, also when their gradients are undefined, so the
+    optimizer learns there that p's gradient is complete (parallel/ddp.py)."""
+    mg = main_grad_of(p)
+    if mg is None or p._backward_hooks:
+        return None
+    hooks = p._post_accumulate_grad_hooks
+    if hooks and len(hooks) > int(hasattr(p, "grad_ready")):
+        return None
+    try:
+        runs = torch._C._will_engine_execute_node(torch.autograd.graph.get_gradient_edge(p).node)
+    except RuntimeError:      # autograd.grad with p among its inputs
+        return None
+    return mg if runs else None
+
+
 def grad_written(p) -> None:
-    """A kernel has added this parameter's gradient to its buffer: lets the optimizer start the reduction of the
-    parameter's bucket (parallel/ddp.py)."""
+    """A kernel of the current stream has added to ``main_grad_target(p)``."""
     p.grad_written = True
-    ready = getattr(p, "grad_ready", None)
-    if ready is not None:
-        ready()
+    if p.is_cuda and hasattr(p, "grad_ready"):
+        p.grad_stream = torch.cuda.current_stream(p.device)
 
 
 def launch_count() -> int:

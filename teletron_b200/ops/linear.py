@@ -19,7 +19,7 @@ import torch
 import torch.nn.functional as F
 
 from . import _lib
-from ._lib import grad_written, main_grad_of
+from ._lib import grad_written, main_grad_target
 from .gemm import EPI_ACCUM, EPI_GATE_RES, EPI_GELU, EPI_NONE, EPI_SILU, gemm
 
 _ACT = {None: EPI_NONE, "gelu": EPI_GELU, "silu": EPI_SILU}
@@ -65,18 +65,21 @@ def _weight_grad(dy, x, w, owner=None):
     mg = getattr(w, "main_grad", None)
     if mg is not None:
         gemm(dy, x, a_mn=True, b_mn=True, out=mg, epi=EPI_ACCUM)
-        grad_written(w)
+        w.grad_written = True
+        ready = getattr(w, "grad_ready", None)
+        if ready is not None:      # lets the optimizer start this parameter's bucket reduction (parallel/ddp.py)
+            ready()
         return None
     return gemm(dy, x, a_mn=True, b_mn=True, out_dtype=w.dtype)
 
 
 def _bias_grad(dy, b):
-    """Column sums of dy: added to the parameter's fp32 gradient buffer when it has one (returns None: no bf16 copy,
-    no accumulation in bf16 over micro-batches, no fold afterwards), else a gradient of the bias' type."""
+    """Column sums of dy: added to the parameter's fp32 gradient buffer where that may take it (returns None: no bf16
+    copy, no accumulation in bf16 over micro-batches, no fold afterwards), else a gradient of the bias' type."""
     if b is None:
         return None
-    mg = main_grad_of(b)
-    if mg is not None and dy.is_cuda and mg.numel() == dy.shape[1]:
+    mg = main_grad_target(b) if dy.is_cuda else None
+    if mg is not None and mg.numel() == dy.shape[1]:
         colsum(dy, add_to=mg.view(-1))
         grad_written(b)
         return None
@@ -222,7 +225,7 @@ class _RowLinear(torch.autograd.Function):
                                             _lib.c_int(B * K), _lib.c_int(0), _lib.stream()), "tt_colsum_partials")
         if ctx.needs_input_grad[1]:
             owner = ctx.w_param
-            mg = main_grad_of(owner)
+            mg = main_grad_target(owner)
             into_main = mg is not None and mg.data_ptr() % 16 == 0
             dw = mg if into_main else torch.empty((N, K), dtype=torch.bfloat16, device=x.device)
             _lib.check(L.tt_rowlin_wgrad(_lib.ptr(dy), _lib.ptr(x), _lib.ptr(dw), _lib.c_int(int(into_main)), *dims,

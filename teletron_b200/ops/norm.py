@@ -41,8 +41,8 @@ def adaln_ref(x, scale, shift, rows_per_batch, eps=1e-6, plus_one=True):
 class _AdaLN(torch.autograd.Function):
     """``with_res``: also return x itself as a second output (an alias) for the residual connection, so that
     the residual's gradient arrives here and is added inside the backward kernel (no separate add kernel).
-    ``owners``: the (weight, bias) parameters behind scale and shift when their gradients go straight into the
-    parameters' fp32 buffers."""
+    ``owners``: the (weight, bias) parameters behind scale and shift, whose gradients go straight into the
+    parameters' fp32 buffers where those may take them."""
 
     @staticmethod
     def forward(ctx, x, scale, shift, rows_per_batch, eps, plus_one, with_res=False, owners=None):
@@ -84,15 +84,15 @@ class _AdaLN(torch.autograd.Function):
         if dres is not None and (dres.dtype != torch.bfloat16 or dres.stride(1) != 1):
             dres = dres.to(torch.bfloat16).contiguous()
         dx = torch.empty((rows, C), dtype=torch.bfloat16, device=x.device)
-        owners = ctx.owners
-        want_mod = (owners is not None or (scale is not None and ctx.needs_input_grad[1])
-                    or (has_shift and ctx.needs_input_grad[2]))
+        targets = None if ctx.owners is None else tuple(_lib.main_grad_target(p) for p in ctx.owners)
+        into_main = targets is not None and None not in targets
+        want_mod = (scale is not None and ctx.needs_input_grad[1]) or (has_shift and ctx.needs_input_grad[2])
         chunks = _chunks(rows_per_batch, batch)
         partial = dmul = dadd = None
         if want_mod:
             partial = torch.empty((batch, chunks, 2, C), dtype=torch.float32, device=x.device)
-            if owners is not None:
-                dmul, dadd = (_lib.main_grad_of(p) for p in owners)
+            if into_main:
+                dmul, dadd = targets
             else:
                 dmul = torch.empty((batch, C), dtype=torch.float32, device=x.device) if scale is not None else None
                 dadd = torch.empty((batch, C), dtype=torch.float32, device=x.device) if has_shift else None
@@ -101,11 +101,11 @@ class _AdaLN(torch.autograd.Function):
             _lib.ptr(rstd), _lib.ptr(scale), _lib.c_ll(mod_ld), _lib.c_int(int(plus_one)), _lib.ptr(dx),
             _lib.c_ll(C), _lib.ptr(dres), _lib.c_ll(dres.stride(0) if dres is not None else 0), _lib.ptr(partial),
             _lib.c_int(chunks),
-            _lib.ptr(dmul), _lib.ptr(dadd), _lib.c_int(int(owners is not None)), _lib.c_int(batch), _lib.c_int(rows_per_batch),
+            _lib.ptr(dmul), _lib.ptr(dadd), _lib.c_int(int(into_main)), _lib.c_int(batch), _lib.c_int(rows_per_batch),
             _lib.c_int(C), _lib.stream())
         _lib.check(rc, "tt_adaln_bwd")
-        if owners is not None:
-            for p in owners:
+        if into_main:
+            for p in ctx.owners:
                 _lib.grad_written(p)
             dmul = dadd = None
         return dx, dmul, dadd, None, None, None, None, None
@@ -130,11 +130,10 @@ def layernorm_affine(x, weight, bias, eps=1e-6, with_res=False):
     """nn.LayerNorm with affine parameters (Wan ``norm3``) through the AdaLN kernel."""
     rows = x.shape[0]
     if (x.is_cuda and weight is not None and bias is not None and torch.is_grad_enabled() and weight.requires_grad
-            and bias.requires_grad and _lib.main_grad_of(weight) is not None and _lib.main_grad_of(bias) is not None):
-        # the parameters stay inputs of the node, so that autograd runs their hooks
+            and bias.requires_grad):
+        # the gradients of w and b lead back to the parameters, also where they stay undefined
         w, b = weight.float().unsqueeze(0), bias.float().unsqueeze(0)
-        out = _AdaLN.apply(x, w, b, rows, eps, False, with_res, (weight, bias))
-        return out
+        return _AdaLN.apply(x, w, b, rows, eps, False, with_res, (weight, bias))
     w = weight.float().unsqueeze(0) if weight is not None else None
     b = bias.float().unsqueeze(0) if bias is not None else None
     if with_res:
@@ -213,7 +212,7 @@ class _RmsRope(torch.autograd.Function):
 def rmsrope_bwd_raw(dy, x, wf, freqs, rstd, D, per_head=False, out=None, owner=None):
     """Backward of rope(rmsnorm(x) * w) from the saved input and rstd: returns (dx bf16, dw fp32 or None).
     ``out``: optional [rows, C] view (any row stride) that receives dx.  ``owner``: the weight parameter; a full-row
-    weight gradient is added to its fp32 buffer when it has one (dw is None then)."""
+    weight gradient is added to its fp32 buffer where that may take it (dw is None then)."""
     rows, C = x.shape
     if dy.stride(1) != 1:
         dy = dy.contiguous()
@@ -232,7 +231,7 @@ def rmsrope_bwd_raw(dy, x, wf, freqs, rstd, D, per_head=False, out=None, owner=N
     _lib.check(rc, "tt_rmsrope_bwd")
     dw = None
     if wf is not None:
-        mg = None if owner is None or per_head else _lib.main_grad_of(owner)
+        mg = None if owner is None or per_head else _lib.main_grad_target(owner)
         dwf = torch.empty((1, C), dtype=torch.float32, device=x.device) if mg is None else mg
         rc = L.tt_colsum_partials(_lib.ptr(partial), _lib.ptr(dwf), _lib.c_int(1), _lib.c_int(ctas),
                                   _lib.c_int(C), _lib.c_int(int(mg is not None)), _lib.stream())

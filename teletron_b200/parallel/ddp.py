@@ -8,7 +8,8 @@ is two objects here:
 
   * ``ParamBuffer`` re-points every parameter into one contiguous bf16 buffer and gives it a
     ``main_grad`` view into one contiguous fp32 buffer.  Weight gradients are accumulated into
-    ``main_grad`` by the wgrad GEMM epilogue; small parameters (biases, norms, modulation) get
+    ``main_grad`` by the wgrad GEMM epilogue, those of biases and full-row norms by the kernels that sum
+    them; the rest (modulation tables, per-head norms, whatever a hook or ``autograd.grad`` wants to see) get
     ordinary ``.grad`` tensors that are folded in by one multi-tensor kernel.  The buffer is laid out
     in up to four regions (weight decay or not, replicated across the tensor-parallel group or not);
     inside a region parameters sit in REVERSE definition order, as in the reference
@@ -296,9 +297,16 @@ class DistributedOptimizer:
     def _install_hooks(self):
         for n, p in self.buf.named:
             p.grad_ready = (lambda name=n: self._param_ready(name))
-            # autograd runs this hook for every parameter of the graph, also with an undefined gradient when the
-            # wgrad GEMM has already accumulated into main_grad (and reported through grad_ready)
-            p.register_post_accumulate_grad_hook(lambda _p, name=n: self._param_ready(name, _p.grad is not None))
+            # autograd runs this hook for every parameter of the graph after all uses of the parameter in the pass,
+            # also with an undefined gradient when kernels have already added to main_grad
+            p.register_post_accumulate_grad_hook(lambda _p, name=n: self._accumulated(name, _p))
+
+    def _accumulated(self, name: str, p: torch.Tensor):
+        written_on = getattr(p, "grad_stream", None)
+        if p.grad is None and written_on is not None and written_on != torch.cuda.current_stream(p.device):
+            # autograd orders streams for gradients that it has seen, not for those that a kernel added to main_grad
+            torch.cuda.current_stream(p.device).wait_stream(written_on)
+        self._param_ready(name, p.grad is not None)
 
     def begin_last_microbatch(self):
         """Arm the gradient-ready hooks: from here on a bucket's reduction starts as soon as every parameter in
