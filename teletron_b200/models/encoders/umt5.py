@@ -16,6 +16,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from ...ops import t5 as t5_ops
+from ...ops._lib import plain_call
 
 
 class T5LayerNorm(nn.Module):
@@ -130,11 +131,7 @@ class UMT5Encoder(nn.Module):
             return False
         if mask is not None and (mask.shape != ids.shape or mask.device != ids.device):
             return False
-        if torch.is_autocast_enabled("cuda") or torch.jit.is_tracing() or torch.compiler.is_compiling():
-            return False
-        if torch.nn.modules.module._has_any_global_hook() or type(ids) is not torch.Tensor:
-            return False
-        if torch._C._functorch.is_functorch_wrapped_tensor(ids):
+        if not plain_call() or torch.nn.modules.module._has_any_global_hook() or type(ids) is not torch.Tensor:
             return False
         grad = torch.is_grad_enabled()
         for m in self.modules():

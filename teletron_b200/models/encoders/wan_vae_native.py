@@ -12,6 +12,7 @@ import torch.nn as nn
 
 from ... import ops
 from ...ops import conv as C
+from ...ops._lib import plain_call
 from . import wan_vae as V
 
 
@@ -29,11 +30,7 @@ def usable(net: nn.Module, x: torch.Tensor) -> bool:
             return False
     elif x.dtype != torch.bfloat16:
         return False
-    if torch.is_autocast_enabled("cuda") or torch.jit.is_tracing() or torch.compiler.is_compiling():
-        return False
-    if type(x) is not torch.Tensor or torch._C._functorch.is_functorch_wrapped_tensor(x):
-        return False
-    if torch.nn.modules.module._has_any_global_hook():
+    if not plain_call() or type(x) is not torch.Tensor or torch.nn.modules.module._has_any_global_hook():
         return False
     grad = torch.is_grad_enabled()
     if grad and x.requires_grad:

@@ -297,14 +297,9 @@ def wan_block_infer(blk: DiTBlock, x2d, context, t_mod, freqs, batch: int, cp):
     for tensors and parameters that are not dense bf16 of one device."""
     if torch.is_grad_enabled() or not x2d.is_cuda or cp is not None or blk.self_attn.head_dim != 128:
         return None
-    if blk.cross_attn.has_image_input or context.dim() != 3 or torch.is_autocast_enabled("cuda"):
+    if blk.cross_attn.has_image_input or context.dim() != 3 or not ops._lib.plain_call():
         return None
-    if torch.jit.is_tracing() or torch.compiler.is_compiling() or torch.nn.modules.module._has_any_global_hook():
-        return None
-    if any(type(t) is not torch.Tensor or torch._C._functorch.is_functorch_wrapped_tensor(t)
-           for t in (x2d, context, t_mod, freqs)):
-        return None
-    if torch.autograd.forward_ad._current_level >= 0:
+    if torch.nn.modules.module._has_any_global_hook() or any(type(t) is not torch.Tensor for t in (x2d, context, t_mod, freqs)):
         return None
     bf16 = torch.bfloat16
     C, dev, (B, Lc, Cc) = blk.dim, x2d.device, context.shape

@@ -118,6 +118,14 @@ def check_status(device: torch.device | None = None) -> None:
                            "results of this step are invalid")
 
 
+def plain_call() -> bool:
+    """Whether a native call may stand in for a chain of torch operators: nothing is on that works on the operators
+    themselves (autocast, tracing, compiling, forward-mode AD, functorch transforms, dispatch modes)."""
+    return not (torch.is_autocast_enabled("cuda") or torch.jit.is_tracing() or torch.compiler.is_compiling()
+                or torch.autograd.forward_ad._current_level >= 0
+                or torch._C._functorch.peek_interpreter_stack() is not None or torch._C._len_torch_dispatch_stack())
+
+
 def main_grad_of(p):
     """The fp32 gradient buffer of a parameter (set by ``parallel.ddp.ParamBuffer``) when kernels may add to it."""
     mg = getattr(p, "main_grad", None)

@@ -1,0 +1,90 @@
+"""What has to keep working where native calls stand in for chains of torch operators."""
+import pytest
+import torch
+import torch.autograd.forward_ad as fwd
+import torch.nn.functional as F
+from torch.utils.flop_counter import FlopCounterMode
+
+from teletron_b200 import ops
+from teletron_b200.models import WanModel, wan_config
+from teletron_b200.models.encoders import UMT5Encoder, WanVideoVAE, wan_vae_native
+from teletron_b200.models.hunyuan import HunyuanVideoModel, hunyuan_config
+from teletron_b200.ops import _lib
+
+pytestmark = pytest.mark.gpu
+BF16 = torch.bfloat16
+
+
+def _vae(dtype=torch.float32):
+    torch.manual_seed(0)
+    return WanVideoVAE(dim=16).to("cuda", dtype).eval()
+
+
+def _t5():
+    torch.manual_seed(0)
+    enc = UMT5Encoder(vocab=50, dim=64, dim_attn=64, dim_ffn=128, num_heads=4, num_layers=1)
+    return enc.to("cuda", BF16).eval().requires_grad_(False), torch.randint(1, 50, (1, 8), device="cuda")
+
+
+def _wan():
+    torch.manual_seed(0)
+    cfg = wan_config("wan2.1-1.3b-t2v", dim=256, num_heads=2, num_layers=1, ffn_dim=640)
+    with torch.device("cuda"):
+        m = WanModel(cfg).to(BF16).eval()
+    x = torch.randn(24, 256, device="cuda", dtype=BF16)
+    return m.blocks[0], (x, torch.randn(1, 16, 256, device="cuda", dtype=BF16), torch.randn(1, 6, 256, device="cuda"),
+                         torch.randn(24, 64, 2, device="cuda"), 1, None)
+
+
+def _single():
+    torch.manual_seed(0)
+    cfg = hunyuan_config("hunyuan-tiny", num_layers=1, num_single_layers=1)
+    with torch.device("cuda"):
+        m = HunyuanVideoModel(cfg).to(BF16).eval()
+    x = torch.randn(24, cfg.hidden_size, device="cuda", dtype=BF16)
+    return m.single_transformer_blocks[0], (x, 16, torch.randn(1, cfg.hidden_size, device="cuda"),
+                                            torch.randn(16, 64, 2, device="cuda"), 1, None)
+
+
+@torch.no_grad()
+def _routes():
+    """The five routes' answers: whether each would run natively now."""
+    from teletron_b200.models import wan
+
+    vae, (enc, ids), (blk, args), (single, sargs) = _vae(), _t5(), _wan(), _single()
+    before = _lib.launch_count()
+    ops.row_linear(torch.randn(1, 64, device="cuda"), torch.randn(8, 64, device="cuda").to(BF16))
+    rows = _lib.launch_count() > before
+    return [wan_vae_native.usable(vae.model.encoder, torch.randn(1, 3, 1, 16, 16, device="cuda")), enc._native(ids, None),
+            wan.wan_block_infer(blk, *args) is not None, single.packs(*sargs), rows]
+
+
+def test_routes_are_native():
+    assert all(_routes())
+
+
+def test_forward_mode():
+    with fwd.dual_level():
+        assert not any(_routes())
+        vae = _vae()
+        x, dx = (torch.randn(3, 1, 16, 16, device="cuda") for _ in range(2))
+        z = fwd.unpack_dual(vae.encode([fwd.make_dual(x, dx)])).tangent
+        h, x, dx, vae = 1e-4, x.double(), dx.double(), vae.double()
+        num = (vae.encode([x + h * dx]) - vae.encode([x - h * dx])) / (2 * h)
+        # TF32 products (2^-11 each way) through about twenty layers
+        assert z is not None and ((z[0] - num[0]).norm() / num.norm()).item() < 0.02
+        w = torch.randn(8, 64, device="cuda").to(BF16)
+        x, dx = (torch.randn(2, 64, device="cuda") for _ in range(2))
+        y = fwd.unpack_dual(ops.row_linear(fwd.make_dual(x, dx), w)).tangent
+        torch.testing.assert_close(y, F.linear(dx, w.float()))
+
+
+def test_vmap_and_operator_counts():
+    w, x = torch.randn(8, 64, device="cuda").to(BF16), torch.randn(3, 1, 64, device="cuda")
+    y = torch.func.vmap(lambda r: ops.row_linear(r, w))(x)
+    torch.testing.assert_close(y, F.linear(x, w.float()))
+    vae = _vae(BF16)
+    with FlopCounterMode(display=False) as count:
+        vae.encode([torch.randn(3, 1, 16, 16, device="cuda", dtype=BF16)])
+    # a 16 x 16 frame through the first residual block alone: two 3 x 3 x 3 convolutions of 16 channels
+    assert count.get_total_flops() > 2 * 2 * 256 * 16 * 16 * 27
