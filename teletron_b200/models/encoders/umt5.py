@@ -125,13 +125,11 @@ class UMT5Encoder(nn.Module):
         w = self.token_embedding.weight
         if not (ids.is_cuda and w.dtype == torch.bfloat16 and ids.dim() == 2 and ids.numel() > 0 and ids.shape[1] <= 4096):
             return False
-        if ids.device.index != torch.cuda.current_device():      # kernels launch on the current device
-            return False
         if self.pos_embedding is not None or self.dim % 8 or self.dim > 8192 or len(self.blocks) == 0:
             return False
         if mask is not None and (mask.shape != ids.shape or mask.device != ids.device):
             return False
-        if not plain_call() or torch.nn.modules.module._has_any_global_hook() or type(ids) is not torch.Tensor:
+        if not plain_call(ids.device) or torch.nn.modules.module._has_any_global_hook() or type(ids) is not torch.Tensor:
             return False
         grad = torch.is_grad_enabled()
         for m in self.modules():

@@ -22,15 +22,13 @@ def usable(net: nn.Module, x: torch.Tensor) -> bool:
     of 16 up to 384 behind the first convolution."""
     if not (x.is_cuda and x.dim() == 5 and x.shape[0] == 1 and x.numel() > 0):
         return False
-    if x.device.index != torch.cuda.current_device():          # kernels launch on the current device
-        return False
     if x.dtype == torch.float32:
         # the per-operator setting: `allow_tf32` may not be read once a program uses it, and follows it otherwise
         if not (torch.backends.cudnn.enabled and torch.backends.cudnn.conv.fp32_precision == "tf32"):
             return False
     elif x.dtype != torch.bfloat16:
         return False
-    if not plain_call() or type(x) is not torch.Tensor or torch.nn.modules.module._has_any_global_hook():
+    if not plain_call(x.device) or type(x) is not torch.Tensor or torch.nn.modules.module._has_any_global_hook():
         return False
     grad = torch.is_grad_enabled()
     if grad and x.requires_grad:

@@ -440,7 +440,7 @@ class SingleStreamBlock(nn.Module):
         128, both streams present, and nothing that would notice the skipped inner modules."""
         if torch.is_grad_enabled() or not x.is_cuda or B != 1 or (cp is not None and cp.size > 1) or self.attn.tp.size > 1:
             return False
-        if not ops._lib.plain_call() or any(type(t) is not torch.Tensor for t in (x, temb, freqs)):
+        if not ops._lib.plain_call(x.device) or any(type(t) is not torch.Tensor for t in (x, temb, freqs)):
             return False
         C = x.shape[1]
         if self.attn.D != 128 or self.attn.heads_local * 128 != C or not 0 < n_video < x.shape[0] or not x.is_contiguous():

@@ -297,7 +297,7 @@ def wan_block_infer(blk: DiTBlock, x2d, context, t_mod, freqs, batch: int, cp):
     for tensors and parameters that are not dense bf16 of one device."""
     if torch.is_grad_enabled() or not x2d.is_cuda or cp is not None or blk.self_attn.head_dim != 128:
         return None
-    if blk.cross_attn.has_image_input or context.dim() != 3 or not ops._lib.plain_call():
+    if blk.cross_attn.has_image_input or context.dim() != 3 or not ops._lib.plain_call(x2d.device):
         return None
     if torch.nn.modules.module._has_any_global_hook() or any(type(t) is not torch.Tensor for t in (x2d, context, t_mod, freqs)):
         return None

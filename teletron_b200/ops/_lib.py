@@ -118,9 +118,12 @@ def check_status(device: torch.device | None = None) -> None:
                            "results of this step are invalid")
 
 
-def plain_call() -> bool:
-    """Whether a native call may stand in for a chain of torch operators: nothing is on that works on the operators
-    themselves (autocast, tracing, compiling, forward-mode AD, functorch transforms, dispatch modes)."""
+def plain_call(device: torch.device) -> bool:
+    """Whether a native call on tensors of ``device`` may stand in for a chain of torch operators: it is the current GPU,
+    which kernels are launched on, and nothing is on that works on the operators themselves (autocast, tracing,
+    compiling, forward-mode AD, functorch transforms, dispatch modes)."""
+    if device.type != "cuda" or device.index != torch.cuda.current_device():
+        return False
     return not (torch.is_autocast_enabled("cuda") or torch.jit.is_tracing() or torch.compiler.is_compiling()
                 or torch.autograd.forward_ad._current_level >= 0
                 or torch._C._functorch.peek_interpreter_stack() is not None or torch._C._len_torch_dispatch_stack())

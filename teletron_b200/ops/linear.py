@@ -244,7 +244,8 @@ def row_linear(x, w, b=None):
     fp32 copies."""
     if (x.is_cuda and x.dim() == 2 and 1 <= x.shape[0] <= _ROWLIN_MAX and w.dim() == 2 and w.dtype == torch.bfloat16
             and x.shape[1] == w.shape[1] and w.shape[1] % 8 == 0 and w.is_contiguous() and w.data_ptr() % 16 == 0
-            and x.device == w.device and x.device.index == torch.cuda.current_device() and (b is None or (b.dtype == torch.bfloat16 and b.is_contiguous()))
-            and _lib.plain_call() and all(type(t) in (torch.Tensor, torch.nn.Parameter) for t in (x, w, b) if t is not None)):
+            and x.device == w.device and (b is None or (b.dtype == torch.bfloat16 and b.is_contiguous()))
+            and all(type(t) in (torch.Tensor, torch.nn.Parameter) for t in (x, w, b) if t is not None)
+            and _lib.plain_call(x.device)):
         return _RowLinear.apply(x.float(), w, b)
     return F.linear(x.float(), w.float(), None if b is None else b.float())

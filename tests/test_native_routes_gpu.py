@@ -6,7 +6,7 @@ import torch.nn.functional as F
 from torch.utils.flop_counter import FlopCounterMode
 
 from teletron_b200 import ops
-from teletron_b200.models import WanModel, wan_config
+from teletron_b200.models import WanModel, wan, wan_config
 from teletron_b200.models.encoders import UMT5Encoder, WanVideoVAE, wan_vae_native
 from teletron_b200.models.hunyuan import HunyuanVideoModel, hunyuan_config
 from teletron_b200.ops import _lib
@@ -49,8 +49,6 @@ def _single():
 @torch.no_grad()
 def _routes():
     """The five routes' answers: whether each would run natively now."""
-    from teletron_b200.models import wan
-
     vae, (enc, ids), (blk, args), (single, sargs) = _vae(), _t5(), _wan(), _single()
     before = _lib.launch_count()
     ops.row_linear(torch.randn(1, 64, device="cuda"), torch.randn(8, 64, device="cuda").to(BF16))
@@ -88,3 +86,13 @@ def test_vmap_and_operator_counts():
         vae.encode([torch.randn(3, 1, 16, 16, device="cuda", dtype=BF16)])
     # a 16 x 16 frame through the first residual block alone: two 3 x 3 x 3 convolutions of 16 channels
     assert count.get_total_flops() > 2 * 2 * 256 * 16 * 16 * 27
+
+
+def test_another_device_is_current(monkeypatch):
+    """Kernels are launched on the current device: tensors of another one take the torch operators."""
+    dev = torch.cuda.current_device
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: dev() + 1)
+    vae, (enc, ids), (blk, args), (single, sargs) = _vae(), _t5(), _wan(), _single()
+    with torch.no_grad():
+        assert wan.wan_block_infer(blk, *args) is None and not single.packs(*sargs) and not enc._native(ids, None)
+        assert not wan_vae_native.usable(vae.model.encoder, torch.randn(1, 3, 1, 16, 16, device="cuda"))
