@@ -51,6 +51,13 @@ def usable(net: nn.Module, x: torch.Tensor) -> bool:
     return True
 
 
+def _gamma(norm: nn.Module) -> torch.Tensor:
+    """The norm's weights as a vector that starts on 16 bytes, as the kernel reads it; parameters may be views into one
+    flat buffer."""
+    g = norm.gamma.detach().reshape(-1)
+    return g if g.data_ptr() % 16 == 0 else g.clone()
+
+
 def open_run(net: nn.Module, x: torch.Tensor):
     return Run() if usable(net, x) else None
 
@@ -88,7 +95,7 @@ class Run:
 
     def norm_conv(self, norm, m, x, res=None, planar=False):
         buf, view, t_off = self._with_history(m, x.shape, x)
-        C.chan_norm(x, norm.gamma.detach().reshape(-1), view)
+        C.chan_norm(x, _gamma(norm), view)
         self._keep_history(m, buf)
         return self.conv(m, C.CONV_SPATIAL, buf, x.shape[0], x.shape[2:4], t_off=t_off, res=res, planar=planar)
 
@@ -117,7 +124,7 @@ class Run:
         n, c = h * w, chunks * e
         if x.dtype != torch.bfloat16 or n > 32768:
             return C.from_planar(m(C.to_planar(x).unsqueeze(0)).squeeze(0))
-        y = C.chan_norm(x, m.norm.gamma.detach().reshape(-1), torch.empty_like(x), act=False)
+        y = C.chan_norm(x, _gamma(m.norm), torch.empty_like(x), act=False)
         qkv = self.conv(m.to_qkv, C.CONV_POINT, y, t, (h, w))
         padded = -(-n // 8) * 8                            # keys in whole vectors; the softmax stops at n
         rows = qkv.new_zeros((t, padded, 3 * c))

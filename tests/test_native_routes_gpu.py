@@ -96,3 +96,17 @@ def test_another_device_is_current(monkeypatch):
     with torch.no_grad():
         assert wan.wan_block_infer(blk, *args) is None and not single.packs(*sargs) and not enc._native(ids, None)
         assert not wan_vae_native.usable(vae.model.encoder, torch.randn(1, 3, 1, 16, 16, device="cuda"))
+
+
+@pytest.mark.parametrize("dtype", [BF16, torch.float32])
+def test_vae_with_parameters_in_one_flat_buffer(dtype):
+    """Views that start anywhere: the same bits as parameters of their own."""
+    vae = _vae(dtype)
+    x = torch.randn(3, 1, 24, 40, device="cuda").to(dtype)
+    ref = vae.encode([x])
+    flat, at = torch.empty(1 + sum(p.numel() for p in vae.parameters()), device="cuda", dtype=dtype), 1
+    for p in vae.parameters():
+        p.data = flat[at:at + p.numel()].copy_(p.data.reshape(-1)).view(p.shape)
+        at += p.numel()
+    assert any(p.data_ptr() % 16 for p in vae.parameters())
+    assert wan_vae_native.usable(vae.model.encoder, x[None]) and torch.equal(vae.encode([x]), ref)
