@@ -200,6 +200,8 @@ class _RowLinear(torch.autograd.Function):
     def forward(ctx, x, w, b):
         B, (N, K) = x.shape[0], w.shape
         x = x.contiguous()
+        if x.data_ptr() % 16:          # a slice at an odd offset
+            x = x.clone()
         y = torch.empty((B, N), dtype=torch.float32, device=x.device)
         _lib.check(_lib.lib().tt_rowlin_fwd(_lib.ptr(x), _lib.ptr(w), _lib.ptr(b), _lib.ptr(y), _lib.c_int(B), _lib.c_int(N),
                                             _lib.c_int(K), _lib.stream()), "tt_rowlin_fwd")

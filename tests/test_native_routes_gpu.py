@@ -110,3 +110,17 @@ def test_vae_with_parameters_in_one_flat_buffer(dtype):
         at += p.numel()
     assert any(p.data_ptr() % 16 for p in vae.parameters())
     assert wan_vae_native.usable(vae.model.encoder, x[None]) and torch.equal(vae.encode([x]), ref)
+
+
+def test_row_linear_of_a_slice():
+    """A contiguous row that does not start on 16 bytes, forward and backward."""
+    torch.manual_seed(1)
+    t = torch.randn(1, 257, device="cuda", requires_grad=True)
+    w = torch.nn.Parameter(torch.randn(24, 256, device="cuda").to(BF16))
+    x = t[:, 1:]
+    assert x.is_contiguous() and x.data_ptr() % 16
+    y = ops.row_linear(x, w)
+    y.backward(torch.ones_like(y))
+    torch.testing.assert_close(y, F.linear(x, w.float()), rtol=1e-5, atol=1e-4)
+    torch.testing.assert_close(t.grad[:, 1:], w.float().sum(0, keepdim=True), rtol=1e-5, atol=1e-4)
+    torch.testing.assert_close(w.grad, x.detach().to(BF16).expand(24, -1))
