@@ -133,7 +133,7 @@ class Run:
         for f in range(t):
             q, k, v = rows[f, :n, :c], rows[f, :, c:2 * c], rows[f, :, 2 * c:]
             scores = ops.gemm(q, k, out_dtype=torch.float32, alpha=c ** -0.5)
-            ops.gemm(C.softmax_split(scores, n), torch.cat([v, v]), b_mn=True, out=out[f])
+            ops.gemm(C.softmax_split(scores, n, 3), torch.cat([v, v, v]), b_mn=True, out=out[f])
         o = C.from_planar(out.view(t, h, w, c).permute(3, 0, 1, 2))
         return self.conv(m.proj, C.CONV_POINT, o, t, (h, w), res=x)
 

@@ -135,12 +135,12 @@ def rounded(x, out=None):
     return _move(x, 2, tuple(x.shape), out)
 
 
-def softmax_split(scores, n: int):
-    """Row softmax of the first ``n`` columns of fp32 [rows, np] as bf16 [rows, 2 np]: high parts, then remainders
-    (zero past column n)."""
+def softmax_split(scores, n: int, parts: int = 2):
+    """Row softmax of the first ``n`` columns of fp32 [rows, np] as bf16 [rows, parts * np] (zero past column n): the
+    rounded values, then the rounded remainders.  Two parts keep 16 bits of a probability, three all of an fp32 one."""
     rows, padded = scores.shape
     assert scores.dtype == torch.float32 and scores.is_contiguous()
-    out = torch.empty((rows, 2 * padded), dtype=torch.bfloat16, device=scores.device)
+    out = torch.empty((rows, parts * padded), dtype=torch.bfloat16, device=scores.device)
     _lib.check(_lib.lib().tt_softmax_split(_lib.ptr(scores), _lib.ptr(out), _lib.c_ll(rows), _lib.c_int(n),
-                                           _lib.c_int(padded), _lib.stream()), "tt_softmax_split")
+                                           _lib.c_int(padded), _lib.c_int(parts), _lib.stream()), "tt_softmax_split")
     return out

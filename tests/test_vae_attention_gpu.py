@@ -1,0 +1,45 @@
+"""Attention of the native VAE (csrc/softmax.cu around two GEMMs): fp32 probabilities, any number of pixels."""
+import pytest
+import torch
+
+from teletron_b200.models.encoders import wan_vae, wan_vae_native
+from teletron_b200.ops import conv as C
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("rows,n", [(3, 1), (5, 8), (64, 1023), (7, 6240)])
+def test_three_parts_are_the_fp32_probability(rows, n):
+    torch.manual_seed(0)
+    padded = -(-n // 8) * 8
+    s = torch.randn(rows, padded, device="cuda") * 4
+    s[:, n:] = float("nan")                                   # not read
+    p = C.softmax_split(s, n, 3).view(rows, 3, padded).double().sum(1)
+    ref = torch.softmax(s[:, :n].double(), dim=1)
+    assert (p[:, n:] == 0).all()
+    # fp32 exponential, sum and product: a few times 2^-24; two parts leave 2^-18
+    assert torch.equal(p, p.float().double())
+    assert ((p[:, :n] - ref).norm() / ref.norm()).item() < 2 ** -21
+
+
+@pytest.mark.parametrize("h,w", [(8, 16), (24, 40)])
+def test_attention_multiplies_fp32_probabilities(monkeypatch, h, w):
+    """The operands of the product with the values: all 24 bits of every probability."""
+    torch.manual_seed(1)
+    n, c, seen = h * w, 64, []
+    m = wan_vae.AttentionBlock(c).to("cuda", torch.bfloat16).requires_grad_(False)
+    gemm = wan_vae_native.ops.gemm
+
+    def spy(a, b, **kw):
+        if kw.get("b_mn"):
+            seen.append((a, b))
+        return gemm(a, b, **kw)
+
+    monkeypatch.setattr(wan_vae_native.ops, "gemm", spy)
+    x = torch.randn(c, 1, h, w, device="cuda").to(torch.bfloat16)
+    wan_vae_native.Run().attention(m, C.from_planar(x))
+    p, v = seen[0]
+    parts = p.shape[1] // n
+    prob = p.view(n, parts, n).double().sum(1)
+    assert torch.equal(v, v[:n].repeat(parts, 1)) and ((prob.sum(1) - 1).abs() < 2 ** -20).all()
+    assert parts == 3 and torch.equal(prob, prob.float().double())
