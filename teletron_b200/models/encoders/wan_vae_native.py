@@ -62,6 +62,11 @@ def open_run(net: nn.Module, x: torch.Tensor):
     return Run() if usable(net, x) else None
 
 
+# Attention scores that are held at a time: 1 GiB in fp32 and 1.5 GiB of probabilities, query rows in whole row tiles.  All
+# 6,240 rows of a 480P frame fit; the library holds all scores of a frame and their softmax, 2 x 4.3 GB at 1080P.
+SCORES = 1 << 28
+
+
 class Run:
     """One encode / decode call: the packed weights, shared by its chunks and tiles."""
 
@@ -122,7 +127,7 @@ class Run:
         """Single-head attention over the pixels of each frame (heads of up to 384 channels)."""
         t, chunks, h, w, e = x.shape
         n, c = h * w, chunks * e
-        if x.dtype != torch.bfloat16 or n > 32768:
+        if x.dtype != torch.bfloat16:
             return C.from_planar(m(C.to_planar(x).unsqueeze(0)).squeeze(0))
         y = C.chan_norm(x, _gamma(m.norm), torch.empty_like(x), act=False)
         qkv = self.conv(m.to_qkv, C.CONV_POINT, y, t, (h, w))
@@ -130,10 +135,13 @@ class Run:
         rows = qkv.new_zeros((t, padded, 3 * c))
         rows[:, :n].unflatten(1, (h, w)).unflatten(3, (3 * chunks, e)).copy_(qkv.permute(0, 2, 3, 1, 4))
         out = torch.empty((t, n, c), dtype=x.dtype, device=x.device)
+        step = max(256, SCORES // padded // 256 * 256)
         for f in range(t):
-            q, k, v = rows[f, :n, :c], rows[f, :, c:2 * c], rows[f, :, 2 * c:]
-            scores = ops.gemm(q, k, out_dtype=torch.float32, alpha=c ** -0.5)
-            ops.gemm(C.softmax_split(scores, n, 3), torch.cat([v, v, v]), b_mn=True, out=out[f])
+            k, v = rows[f, :, c:2 * c], rows[f, :, 2 * c:]
+            v = torch.cat([v, v, v])
+            for i in range(0, n, step):
+                scores = ops.gemm(rows[f, i:min(i + step, n), :c], k, out_dtype=torch.float32, alpha=c ** -0.5)
+                ops.gemm(C.softmax_split(scores, n, 3), v, b_mn=True, out=out[f, i:i + step])
         o = C.from_planar(out.view(t, h, w, c).permute(3, 0, 1, 2))
         return self.conv(m.proj, C.CONV_POINT, o, t, (h, w), res=x)
 

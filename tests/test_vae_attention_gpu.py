@@ -43,3 +43,26 @@ def test_attention_multiplies_fp32_probabilities(monkeypatch, h, w):
     prob = p.view(n, parts, n).double().sum(1)
     assert torch.equal(v, v[:n].repeat(parts, 1)) and ((prob.sum(1) - 1).abs() < 2 ** -20).all()
     assert parts == 3 and torch.equal(prob, prob.float().double())
+
+
+@pytest.mark.parametrize("t,h,w,scores", [(1, 192, 193, None), (2, 30, 53, 1 << 19), (1, 17, 16, 1)])
+def test_query_rows_in_blocks(monkeypatch, t, h, w, scores):
+    """Frames whose scores exceed what is held at a time (the first by its real size), against fp64."""
+    torch.manual_seed(2)
+    if scores is not None:
+        monkeypatch.setattr(wan_vae_native, "SCORES", scores)
+    m = wan_vae.AttentionBlock(64)
+    torch.nn.init.normal_(m.proj.weight, std=0.1)
+    m = m.to("cuda", torch.bfloat16).requires_grad_(False)
+    x = torch.randn(64, t, h, w, device="cuda").to(torch.bfloat16)
+    xb = C.from_planar(x)
+    torch.cuda.reset_peak_memory_stats()
+    held = torch.cuda.memory_allocated()
+    out = C.to_planar(wan_vae_native.Run().attention(m, xb))
+    assert torch.cuda.max_memory_allocated() - held < 3 * 2 ** 30
+    old = m(x[None])[0]
+    m, ref = m.double(), torch.empty(64, t, h, w, device="cuda", dtype=torch.float64)
+    for f in range(t):
+        ref[:, f:f + 1] = m(x[None, :, f:f + 1].double())[0]
+    e_new, e_old = (((a.double() - ref).norm() / ref.norm()).item() for a in (out, old))
+    assert e_new <= e_old * 1.05 + 1e-5, (e_new, e_old)
