@@ -271,7 +271,7 @@ class DiTBlock(nn.Module):
         out = wan_block_infer(self, x2d, context, t_mod, freqs, batch, cp)
         if out is not None:
             return out
-        e = t_mod + self.modulation  # [B, 6, C] fp32 (the bf16 table is widened inside the add)
+        e = t_mod.float() + self.modulation  # [B, 6, C] fp32 (the bf16 table is widened inside the add)
         # each norm also hands back its input for the residual branch, so that the residual's gradient is added
         # inside the norm's backward kernel
         h, xr = ops.adaln_res(x2d, e[:, 1], e[:, 0], rows_per_batch, self.eps)
