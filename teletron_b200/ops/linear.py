@@ -199,9 +199,6 @@ class _RowLinear(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w, b):
         B, (N, K) = x.shape[0], w.shape
-        x = x.contiguous()
-        if x.data_ptr() % 16:          # a slice at an odd offset
-            x = x.clone()
         y = torch.empty((B, N), dtype=torch.float32, device=x.device)
         _lib.check(_lib.lib().tt_rowlin_fwd(_lib.ptr(x), _lib.ptr(w), _lib.ptr(b), _lib.ptr(y), _lib.c_int(B), _lib.c_int(N),
                                             _lib.c_int(K), _lib.stream()), "tt_rowlin_fwd")
@@ -212,6 +209,11 @@ class _RowLinear(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         x, w = ctx.saved_tensors
+        if torch.is_grad_enabled():    # create_graph: gradients of the gradients are wanted
+            dx = dy @ w.float() if ctx.needs_input_grad[0] else None
+            dw = (dy.t() @ x).to(w.dtype) if ctx.needs_input_grad[1] else None
+            db = dy.sum(0).to(ctx.bias_dtype) if ctx.bias_dtype is not None and ctx.needs_input_grad[2] else None
+            return dx, dw, db
         dy = dy.contiguous()
         B, (N, K) = x.shape[0], w.shape
         L = _lib.lib()
@@ -249,5 +251,8 @@ def row_linear(x, w, b=None):
             and x.device == w.device and (b is None or (b.dtype == torch.bfloat16 and b.is_contiguous()))
             and all(type(t) in (torch.Tensor, torch.nn.Parameter) for t in (x, w, b) if t is not None)
             and _lib.plain_call(x.device)):
-        return _RowLinear.apply(x.float(), w, b)
+        x = x.float().contiguous()
+        if x.data_ptr() % 16:          # a slice at an odd offset
+            x = x.clone()
+        return _RowLinear.apply(x, w, b)
     return F.linear(x.float(), w.float(), None if b is None else b.float())

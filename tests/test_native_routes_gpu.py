@@ -124,3 +124,18 @@ def test_row_linear_of_a_slice():
     torch.testing.assert_close(y, F.linear(x, w.float()), rtol=1e-5, atol=1e-4)
     torch.testing.assert_close(t.grad[:, 1:], w.float().sum(0, keepdim=True), rtol=1e-5, atol=1e-4)
     torch.testing.assert_close(w.grad, x.detach().to(BF16).expand(24, -1))
+
+
+def test_row_linear_second_derivatives():
+    torch.manual_seed(2)
+    x = torch.randn(2, 64, device="cuda", requires_grad=True)
+    w = torch.nn.Parameter(torch.randn(8, 64, device="cuda").to(BF16))
+    b = torch.nn.Parameter(torch.randn(8, device="cuda").to(BF16))
+
+    def penalty(f):
+        gx, gw, gb = torch.autograd.grad(f().square().sum(), [x, w, b], create_graph=True)
+        return torch.autograd.grad(gx.square().sum() + gw.float().square().sum() + gb.float().sum(), [x, w, b])
+
+    got = penalty(lambda: ops.row_linear(x, w, b))
+    for g, r in zip(got, penalty(lambda: F.linear(x, w.float(), b.float()))):
+        torch.testing.assert_close(g, r, rtol=1e-2, atol=1e-2 * r.abs().max().item())   # bf16 gradients
