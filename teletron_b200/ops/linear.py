@@ -248,7 +248,8 @@ def row_linear(x, w, b=None):
     fp32 copies."""
     if (x.is_cuda and x.dim() == 2 and 1 <= x.shape[0] <= _ROWLIN_MAX and w.dim() == 2 and w.dtype == torch.bfloat16
             and x.shape[1] == w.shape[1] and w.shape[1] % 8 == 0 and w.is_contiguous() and w.data_ptr() % 16 == 0
-            and x.device == w.device and (b is None or (b.dtype == torch.bfloat16 and b.is_contiguous()))
+            and x.device == w.device and w.numel() > 0
+            and (b is None or (b.dtype == torch.bfloat16 and b.is_contiguous() and b.shape == w.shape[:1] and b.device == w.device))
             and all(type(t) in (torch.Tensor, torch.nn.Parameter) for t in (x, w, b) if t is not None)
             and _lib.plain_call(x.device)):
         x = x.float().contiguous()

@@ -139,3 +139,15 @@ def test_row_linear_second_derivatives():
     got = penalty(lambda: ops.row_linear(x, w, b))
     for g, r in zip(got, penalty(lambda: F.linear(x, w.float(), b.float()))):
         torch.testing.assert_close(g, r, rtol=1e-2, atol=1e-2 * r.abs().max().item())   # bf16 gradients
+
+
+def test_row_linear_refuses_what_linear_refuses():
+    """A bias of another length or device is an error; no weights is an empty result."""
+    x, w = torch.randn(2, 64, device="cuda"), torch.randn(8, 64, device="cuda").to(BF16)
+    for b in (torch.zeros(5, device="cuda", dtype=BF16), torch.zeros(8, dtype=BF16)):
+        with pytest.raises(RuntimeError):
+            ops.row_linear(x, w, b)
+    assert ops.row_linear(x, w[:0]).shape == (2, 0)
+    # a bias that broadcasts, as F.linear has it
+    b = torch.ones(1, device="cuda", dtype=BF16)
+    torch.testing.assert_close(ops.row_linear(x, w, b), F.linear(x, w.float(), b.float()))
