@@ -303,7 +303,7 @@ def wan_block_infer(blk: DiTBlock, x2d, context, t_mod, freqs, batch: int, cp):
         return None
     bf16 = torch.bfloat16
     C, dev, (B, Lc, Cc) = blk.dim, x2d.device, context.shape
-    if x2d.dtype != bf16 or x2d.dim() != 2 or x2d.stride(1) != 1 or x2d.stride(0) % 8 or x2d.shape[0] % batch:
+    if x2d.dtype != bf16 or x2d.dim() != 2 or x2d.shape[1] != C or x2d.stride(1) != 1 or x2d.stride(0) % 8 or x2d.shape[0] % batch:
         return None
     if context.dtype != bf16 or not context.is_contiguous() or (B, Cc) != (batch, C) or context.device != dev:
         return None
@@ -311,13 +311,15 @@ def wan_block_infer(blk: DiTBlock, x2d, context, t_mod, freqs, batch: int, cp):
         return None
     if freqs.dtype != torch.float32 or not freqs.is_contiguous() or freqs.shape[1:] != (64, 2) or freqs.device != dev:
         return None
-    params = _block_params(blk)
-    for p in params:
-        if p is None or p.dtype != bf16 or p.device != dev or not p.is_contiguous():
+    params, F_ = _block_params(blk), blk.ffn[0].weight.shape[0]
+    shapes = ((1, 6, C), (3 * C, C), (3 * C,), (C,), (C,), (C, C), (C,), (C,), (C,), (C, C), (C,), (2 * C, C), (2 * C,), (C,),
+              (C,), (C, C), (C,), (F_, C), (F_,), (C, F_), (C,))
+    for p, shape in zip(params, shapes):
+        if p is None or p.dtype != bf16 or p.device != dev or p.shape != shape or not p.is_contiguous():
             return None
     if any(m._forward_hooks or m._forward_pre_hooks for m in blk.modules() if m is not blk):
         return None
-    lib, S, F_ = ops._lib, x2d.shape[0] // batch, blk.ffn[0].weight.shape[0]
+    lib, S = ops._lib, x2d.shape[0] // batch
     ptrs = [p.data_ptr() for p in params]
     if any(a & 15 for a in ptrs) or (x2d.data_ptr() | context.data_ptr() | freqs.data_ptr()) & 15 or F_ % 8 or S == 0:
         return None

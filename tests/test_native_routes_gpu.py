@@ -151,3 +151,17 @@ def test_row_linear_refuses_what_linear_refuses():
     # a bias that broadcasts, as F.linear has it
     b = torch.ones(1, device="cuda", dtype=BF16)
     torch.testing.assert_close(ops.row_linear(x, w, b), F.linear(x, w.float(), b.float()))
+
+
+def test_block_call_looks_at_the_shapes():
+    """Parameters that do not fit the block go to the op layer, which refuses them."""
+    blk, args = _wan()
+    with torch.no_grad():
+        assert wan.wan_block_infer(blk, *args) is not None
+        for mod, name in ((blk, "modulation"), (blk.self_attn.qkv, "bias"), (blk.ffn[2], "weight"), (blk.cross_attn.norm_k, "weight")):
+            old = getattr(mod, name)
+            setattr(mod, name, torch.nn.Parameter(old.data[..., :-8].contiguous()))
+            assert wan.wan_block_infer(blk, *args) is None
+            setattr(mod, name, old)
+        assert wan.wan_block_infer(blk, args[0][:, :-8], *args[1:]) is None
+        assert wan.wan_block_infer(blk, *args) is not None
