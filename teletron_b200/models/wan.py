@@ -305,7 +305,7 @@ def wan_block_infer(blk: DiTBlock, x2d, context, t_mod, freqs, batch: int, cp):
     C, dev, (B, Lc, Cc) = blk.dim, x2d.device, context.shape
     if x2d.dtype != bf16 or x2d.dim() != 2 or x2d.shape[1] != C or x2d.stride(1) != 1 or x2d.stride(0) % 8 or x2d.shape[0] % batch:
         return None
-    if context.dtype != bf16 or not context.is_contiguous() or (B, Cc) != (batch, C) or context.device != dev:
+    if context.dtype != bf16 or not context.is_contiguous() or (B, Cc) != (batch, C) or Lc == 0 or context.device != dev:
         return None
     if t_mod.dtype != torch.float32 or not t_mod.is_contiguous() or t_mod.shape != (batch, 6, C) or t_mod.device != dev:
         return None

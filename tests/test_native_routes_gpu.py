@@ -165,3 +165,9 @@ def test_block_call_looks_at_the_shapes():
             setattr(mod, name, old)
         assert wan.wan_block_infer(blk, args[0][:, :-8], *args[1:]) is None
         assert wan.wan_block_infer(blk, *args) is not None
+
+
+def test_block_call_leaves_an_empty_context_to_the_op_layer():
+    blk, args = _wan()
+    with torch.no_grad():
+        assert wan.wan_block_infer(blk, args[0], args[1][:, :0], *args[2:]) is None
