@@ -17,6 +17,7 @@ import torch.nn.functional as F
 
 from ...ops import t5 as t5_ops
 from ...ops._lib import plain_call
+from ..native_route import plain_modules
 
 
 class T5LayerNorm(nn.Module):
@@ -108,6 +109,10 @@ class T5SelfAttentionBlock(nn.Module):
         return x + self.ffn(self.norm2(x))
 
 
+_MODULES = (T5SelfAttentionBlock, T5LayerNorm, T5Attention, T5RelativeEmbedding, T5FeedForward, nn.Embedding, nn.Linear,
+            nn.GELU, nn.ModuleList, nn.Sequential)
+
+
 class UMT5Encoder(nn.Module):
     def __init__(self, vocab=256384, dim=4096, dim_attn=4096, dim_ffn=10240, num_heads=64, num_layers=24,
                  num_buckets=32, shared_pos=False):
@@ -129,12 +134,10 @@ class UMT5Encoder(nn.Module):
             return False
         if mask is not None and (mask.shape != ids.shape or mask.device != ids.device):
             return False
-        if not plain_call(ids.device) or torch.nn.modules.module._has_any_global_hook() or type(ids) is not torch.Tensor:
+        if not plain_call(ids.device) or type(ids) is not torch.Tensor or not plain_modules(self, _MODULES, root_hooks=False):
             return False
         grad = torch.is_grad_enabled()
         for m in self.modules():
-            if m is not self and (m._forward_hooks or m._forward_pre_hooks):
-                return False
             for p in m._parameters.values():
                 if p is not None and (p.dtype != torch.bfloat16 or p.device != ids.device or not p.is_contiguous()
                                       or (grad and p.requires_grad) or p.data_ptr() % 16):

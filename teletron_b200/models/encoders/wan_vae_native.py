@@ -13,7 +13,12 @@ import torch.nn as nn
 from ... import ops
 from ...ops import conv as C
 from ...ops._lib import plain_call
+from ..native_route import plain_modules
 from . import wan_vae as V
+
+
+_MODULES = (V.CausalConv3d, V.RMS_norm, V.Resample, V.ResidualBlock, V.AttentionBlock, nn.Conv2d, nn.SiLU, nn.Dropout,
+            nn.Identity, nn.Upsample, nn.ZeroPad2d, nn.Sequential)
 
 
 def usable(net: nn.Module, x: torch.Tensor) -> bool:
@@ -28,15 +33,13 @@ def usable(net: nn.Module, x: torch.Tensor) -> bool:
             return False
     elif x.dtype != torch.bfloat16:
         return False
-    if not plain_call(x.device) or type(x) is not torch.Tensor or torch.nn.modules.module._has_any_global_hook():
+    if not plain_call(x.device) or type(x) is not torch.Tensor or not plain_modules(net, _MODULES):
         return False
     grad = torch.is_grad_enabled()
     if grad and x.requires_grad:
         return False
     first, last = net.conv1, net.head[2]
     for m in net.modules():
-        if m._forward_hooks or m._forward_pre_hooks:
-            return False
         if isinstance(m, nn.Dropout) and m.training and m.p > 0:
             return False
         if isinstance(m, (nn.Conv2d, nn.Conv3d)):

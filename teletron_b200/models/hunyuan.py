@@ -37,6 +37,7 @@ from ..ops.norm import rmsrope_fwd_raw
 from ..parallel import recompute as rc
 from ..parallel.tp import ColumnParallelLinear, FusedColumnParallel, RowParallelLinear, TPContext
 from ..parallel.ulysses import UlyssesContext, _HeadToSeq, _SeqToHead
+from .native_route import plain_modules
 from .registry import MODELS
 
 
@@ -449,9 +450,8 @@ class SingleStreamBlock(nn.Module):
             return False
         if x.dtype != torch.bfloat16 or self.proj_mlp.bias is None or self.proj_out.weight.shape[1] != C + self.proj_mlp.weight.shape[0]:
             return False
-        if torch.nn.modules.module._has_any_global_hook():
-            return False
-        return not any(m._forward_hooks or m._forward_pre_hooks for m in self.modules())
+        return plain_modules(self, (HunyuanAttention, FusedColumnParallel, HeadNorm, AdaNormZero, ColumnParallelLinear,
+                                    SingleProjOut, nn.Linear))
 
 
 class _PairBlock(nn.Module):

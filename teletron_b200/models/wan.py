@@ -31,6 +31,7 @@ from .. import ops
 from ..ops.gemm import pair_gemm
 from ..parallel import recompute as rc
 from ..parallel.ulysses import UlyssesContext
+from .native_route import plain_modules
 
 T5_CONTEXT_TOKENS = 512
 
@@ -291,15 +292,20 @@ def _block_params(blk: DiTBlock):
             ca.norm_k.weight, ca.o.weight, ca.o.bias, f1.weight, f1.bias, f2.weight, f2.bias)
 
 
+_BLOCK_MODULES = (SelfAttention, CrossAttention, FusedProj, RMSNormWeight, nn.Linear, nn.LayerNorm, nn.GELU, nn.Sequential)
+
+
 def wan_block_infer(blk: DiTBlock, x2d, context, t_mod, freqs, batch: int, cp):
     """The block without gradients as one native call (csrc/wan_block.cu), or None where the op layer has to run:
-    with gradients, on CPU, under context parallelism or tracing, with image tokens, with hooks on inner modules, or
+    with gradients, on CPU, under context parallelism or tracing, with image tokens, with hooks on inner modules or modules put in their place, or
     for tensors and parameters that are not dense bf16 of one device."""
     if torch.is_grad_enabled() or not x2d.is_cuda or cp is not None or blk.self_attn.head_dim != 128:
         return None
     if blk.cross_attn.has_image_input or context.dim() != 3 or not ops._lib.plain_call(x2d.device):
         return None
-    if torch.nn.modules.module._has_any_global_hook() or any(type(t) is not torch.Tensor for t in (x2d, context, t_mod, freqs)):
+    if any(type(t) is not torch.Tensor for t in (x2d, context, t_mod, freqs)):
+        return None
+    if not plain_modules(blk, _BLOCK_MODULES, root_hooks=False) or not blk.eps == blk.self_attn.eps == blk.cross_attn.eps:
         return None
     bf16 = torch.bfloat16
     C, dev, (B, Lc, Cc) = blk.dim, x2d.device, context.shape
@@ -317,8 +323,6 @@ def wan_block_infer(blk: DiTBlock, x2d, context, t_mod, freqs, batch: int, cp):
     for p, shape in zip(params, shapes):
         if p is None or p.dtype != bf16 or p.device != dev or p.shape != shape or not p.is_contiguous():
             return None
-    if any(m._forward_hooks or m._forward_pre_hooks for m in blk.modules() if m is not blk):
-        return None
     lib, S = ops._lib, x2d.shape[0] // batch
     ptrs = [p.data_ptr() for p in params]
     if any(a & 15 for a in ptrs) or (x2d.data_ptr() | context.data_ptr() | freqs.data_ptr()) & 15 or F_ % 8 or S == 0:

@@ -10,6 +10,7 @@ def add_norm(x, delta, weight, eps):
     """(x + delta, T5 layer norm of it); delta None: (x, norm of x)."""
     assert x.is_contiguous() and x.dtype == torch.bfloat16 and weight.is_contiguous()
     C = x.shape[-1]
+    assert weight.shape == (C,)
     if delta is not None:
         assert delta.shape == x.shape and delta.is_contiguous() and delta.dtype == torch.bfloat16
     xo = x if delta is None else torch.empty_like(x)

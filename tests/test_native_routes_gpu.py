@@ -171,3 +171,47 @@ def test_block_call_leaves_an_empty_context_to_the_op_layer():
     blk, args = _wan()
     with torch.no_grad():
         assert wan.wan_block_infer(blk, args[0], args[1][:, :0], *args[2:]) is None
+
+
+class _Lora(torch.nn.Module):
+    """A wrapper in the manner of low-rank adapters: shows its base layer's weight and computes something else."""
+
+    def __init__(self, base):
+        super().__init__()
+        self.base = base
+
+    weight = property(lambda self: self.base.weight)
+    bias = property(lambda self: self.base.bias)
+
+    def forward(self, x, **kw):
+        return self.base(x, **kw) * 2
+
+
+def test_modules_put_in_the_place_of_others():
+    """Wrapped layers, instance-level forwards and other epsilons are computed, not skipped."""
+    blk, args = _wan()
+    single, sargs = _single()
+    vae, (enc, ids) = _vae(BF16), _t5()
+    x = torch.randn(3, 1, 16, 16, device="cuda", dtype=BF16)
+
+    def single_out():
+        from teletron_b200.models.hunyuan import _PairBlock
+
+        return _PairBlock(single)(sargs[0], sargs[1], sargs[2], sargs[3], 1, None, None)
+
+    calls = [(lambda: blk(*args), blk.self_attn, "qkv"), (lambda: blk(*args), blk.cross_attn, "kv"),
+             (single_out, single, "proj_mlp"), (lambda: vae.encode([x]), vae.model.encoder.middle[0].residual, "2"),
+             (lambda: enc(ids), enc.blocks[0], "norm1")]
+    with torch.no_grad():
+        for f, owner, name in calls:
+            ref, old = f(), owner._modules[name]
+            owner._modules[name] = _Lora(old)
+            assert not torch.equal(f(), ref), name
+            owner._modules[name] = old
+            own = old.forward
+            old.forward = lambda *a, **kw: own(*a, **kw) * 2
+            assert not torch.equal(f(), ref), name
+            del old.forward
+            assert torch.equal(f(), ref)
+        blk.self_attn.eps = 0.5
+        assert wan.wan_block_infer(blk, *args) is None
