@@ -37,7 +37,7 @@ from ..ops.norm import rmsrope_fwd_raw
 from ..parallel import recompute as rc
 from ..parallel.tp import ColumnParallelLinear, FusedColumnParallel, RowParallelLinear, TPContext
 from ..parallel.ulysses import UlyssesContext, _HeadToSeq, _SeqToHead
-from .native_route import plain_modules
+from .native_route import plain_modules, unobserved
 from .registry import MODELS
 
 
@@ -156,7 +156,10 @@ class FeedForward(nn.Module):
         return self.net[2](h)
 
     def residual(self, x_rows, residual, gate, rows_per_batch):
-        """residual + gate * forward(x_rows), in the second projection's epilogue where it ends in no reduce-scatter."""
+        """residual + gate * forward(x_rows), in the second projection's epilogue where it ends in no reduce-scatter and
+        nobody sees the output of this module or of that projection."""
+        if type(self.net[2]) is not RowParallelLinear or not unobserved(self, self.net[2]):
+            return _gated_residual(self(x_rows), residual, gate, rows_per_batch)
         return _project_out(self.net[2], self.net[0].proj(x_rows, act=self.act), residual, gate, rows_per_batch)
 
 

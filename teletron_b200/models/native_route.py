@@ -17,3 +17,10 @@ def plain_modules(root: nn.Module, types, root_hooks: bool = True) -> bool:
         if "forward" in m.__dict__ or (m is not root and type(m) not in types):
             return False
     return True
+
+
+def unobserved(*modules: nn.Module) -> bool:
+    """True when no hook, forward or backward, and no instance-level forward sits on any of the modules."""
+    return not (_has_any_global_hook() or any(
+        m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks or "forward" in m.__dict__
+        for m in modules))
