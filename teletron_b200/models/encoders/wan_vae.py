@@ -8,9 +8,10 @@ wan_video_vae.py:34-598) so its checkpoints load: ``encoder.conv1``, ``encoder.d
   * one pass over the whole clip (short clips: the 96-channel full-resolution activations of the first stage cost
     about 0.19 GB per 480P frame in bf16);
   * in temporal chunks, as the reference does (wan_video_vae.py:121-173, 215-221, 526-576): the encoder takes the
-    first frame, then ``chunk_frames`` (4) frames at a time, the decoder one latent frame at a time, and every
+    first frame, then ``chunk_frames`` frames at a time, the decoder that many latent frames at a time, and every
     causal convolution keeps the last frames of its input as the history of the next chunk (``StreamState``), so
-    activation memory does not grow with the clip length.
+    activation memory does not grow with the clip length.  On the native kernels the first frame rides with the first
+    chunk.  Default chunks: see ``WanVideoVAE._default_chunk``.
 Temporal resampling:
   * down-sampling keeps the first frame and applies the stride-2, kernel-3 ``time_conv`` to the sequence without
     padding (across chunks: the last frame of the previous chunk is the first input of the next);
@@ -246,7 +247,8 @@ class VideoVAE_(nn.Module):
 
     def encode(self, x, scale, chunk_frames: int = 0, run=None):
         """``chunk_frames`` > 0: the first frame, then that many frames at a time (a multiple of 4), with the
-        convolutions' history carried between chunks.  ``run``: a ``wan_vae_native.Run`` that may compute this pass."""
+        convolutions' history carried between chunks.  ``run``: a ``wan_vae_native.Run`` that may compute this pass; its
+        first chunk holds the first frame too."""
         encoder, first = self.encoder, 1
         # three stride-2 windows need two pixels each
         if run is not None and min(x.shape[3], x.shape[4]) >= 16:
@@ -357,6 +359,19 @@ class WanVideoVAE(nn.Module):
     # 0 = always the whole clip, n = chunks of n frames (encoder; multiple of 4) / n latent frames (decoder)
     whole_clip_frames = 33
 
+    @staticmethod
+    def _default_chunk(native: bool, decoder: bool, height: int, width: int, itemsize: int) -> int:
+        """Frames (decoder: latent frames) per chunk when the caller names none, for frames (tiles) of height x width
+        pixels.  The modules take the reference's 4 and 1.  The native kernels use less memory per frame and run faster on
+        longer chunks, so they take as many as keep the peak at what the modules need: 8 and 2 (480P x 49 in bf16: 3.6
+        GiB and 127 ms, 4 frames 2.5 GiB and 134 ms, modules 3.9 GiB; decoding 480P in fp32: 8.8 GiB, modules 8.9), and 16
+        and 4 for small frames, where launches count (30 x 52 latent tiles: 96 ms instead of 105) and the peak stays
+        below 4.5 GiB."""
+        if not native:
+            return 1 if decoder else 4
+        small = height * width * itemsize <= 1 << 19
+        return (4 if small else 2) if decoder else (16 if small else 8)
+
     def _chunk(self, frames: int, chunk_frames, default: int) -> int:
         if chunk_frames is None:
             return default if frames > self.whole_clip_frames else 0
@@ -369,9 +384,10 @@ class WanVideoVAE(nn.Module):
             x = v.unsqueeze(0).to(device or v.device)
             scale = self._scale(x)
             run = open_run(self.model.encoder, x)
-            ck = self._chunk(x.shape[2], chunk_frames, 4 if run is None else 16)
+            tile = (tile_size[0] * 8, tile_size[1] * 8)
+            hw = (min(n, m) if tiled else n for n, m in zip(x.shape[3:], tile))
+            ck = self._chunk(x.shape[2], chunk_frames, self._default_chunk(run is not None, False, *hw, x.element_size()))
             if tiled:
-                tile = (tile_size[0] * 8, tile_size[1] * 8)
                 stride = (tile_stride[0] * 8, tile_stride[1] * 8)
                 z = self._tiled(lambda t: self.model.encode(t, scale, ck, run), x, tile, stride, 1 / 8, self.z_dim)
             else:
@@ -387,7 +403,9 @@ class WanVideoVAE(nn.Module):
             scale = self._scale(z)
             # bf16 weights are refused by the decoder's enlargement layers, with and without the native kernels
             run = open_run(self.model.decoder, z) if z.dtype == torch.float32 else None
-            ck = self._chunk(4 * (z.shape[2] - 1) + 1, chunk_frames, 1 if run is None else 4)
+            hw = (8 * (min(n, m) if tiled else n) for n, m in zip(z.shape[3:], tile_size))
+            ck = self._chunk(4 * (z.shape[2] - 1) + 1, chunk_frames,
+                             self._default_chunk(run is not None, True, *hw, z.element_size()))
             if tiled:
                 v = self._tiled(lambda t: self.model.decode(t, scale, ck, run), z, tile_size, tile_stride, 8, 3)
             else:

@@ -1,8 +1,9 @@
-"""Attention of the native VAE (csrc/softmax.cu around two GEMMs): fp32 probabilities, any number of pixels."""
+"""The native VAE beyond single kernels: attention (csrc/softmax.cu around two GEMMs: fp32 probabilities, any number of
+pixels) and the memory of its default chunks."""
 import pytest
 import torch
 
-from teletron_b200.models.encoders import wan_vae, wan_vae_native
+from teletron_b200.models.encoders import WanVideoVAE, wan_vae, wan_vae_native
 from teletron_b200.ops import conv as C
 
 pytestmark = pytest.mark.gpu
@@ -66,3 +67,30 @@ def test_query_rows_in_blocks(monkeypatch, t, h, w, scores):
         ref[:, f:f + 1] = m(x[None, :, f:f + 1].double())[0]
     e_new, e_old = (((a.double() - ref).norm() / ref.norm()).item() for a in (out, old))
     assert e_new <= e_old * 1.05 + 1e-5, (e_new, e_old)
+
+
+@pytest.mark.parametrize("decoder", [False, True])
+def test_default_chunks_need_no_more_memory_than_the_modules(monkeypatch, decoder):
+    torch.manual_seed(3)
+    vae = WanVideoVAE().to("cuda", torch.float32 if decoder else torch.bfloat16).eval()
+    x = torch.randn(1, 16, 10, 68, 68, device="cuda") if decoder else torch.rand(1, 3, 37, 544, 544, device="cuda").bfloat16()
+
+    def peak():
+        torch.cuda.empty_cache()
+        torch.cuda.reset_peak_memory_stats()
+        held = torch.cuda.memory_allocated()
+        (vae.decode if decoder else vae.encode)(x)
+        return (torch.cuda.max_memory_allocated() - held) / 2 ** 30
+
+    native = peak()
+    monkeypatch.setattr(wan_vae, "open_run", lambda net, t: None)
+    modules = peak()
+    assert native < modules + 0.2, (native, modules)
+
+
+def test_default_chunks():
+    f = WanVideoVAE._default_chunk
+    assert [f(False, d, 480, 832, 2) for d in (False, True)] == [4, 1]
+    assert [f(True, d, 512, 512, 2) for d in (False, True)] == [16, 4]
+    assert [f(True, d, 512, 520, 2) for d in (False, True)] == [8, 2]
+    assert f(True, True, 240, 416, 4) == 4 and f(True, True, 480, 832, 4) == 2
