@@ -603,11 +603,10 @@ TT_API int tt_colsum_partials(const float* partial, float* out, int groups, int 
 }
 
 // ------------------------------------------------------------------ RMSNorm + RoPE, one row per warp
-// C = NV * 256: each lane holds NV 16-byte vectors of the row (packed: the 10 KB of a 5120-wide row are 80
-// registers per lane), the reductions are
-// warp shuffles (over the 8 or 16 lanes of a head with PER_HEAD), eight rows per CTA are in flight.  The row-per-CTA
-// kernel above reached a third of the copy bandwidth at C = 1536 (two block barriers per 3 KB row), half of it at 3072
-// and 5120.  The weight row lives in shared memory.
+// C = NV * 256: each lane holds NV 16-byte vectors of the row (packed: the 10 KB of a 5120-wide row are 80 registers per
+// lane), the reductions are warp shuffles (over the 8 or 16 lanes of a head with PER_HEAD), eight rows per CTA are in
+// flight.  The row-per-CTA kernel above reached a third of the copy bandwidth at C = 1536 (two block barriers per 3 KB
+// row), half of it at 3072 and 5120.  The weight row lives in shared memory.
 template <int NV, bool PER_HEAD>
 __global__ void __launch_bounds__(NT, 2)
 rmsrope_fwd_warp_kernel(const bf16* __restrict__ in, long long ldi, bf16* __restrict__ out, long long ldo,
@@ -910,7 +909,14 @@ static int rmsrope_fwd_impl(const void* x, long long ldx, void* y, long long ldy
   TT_CHECK(freqs == nullptr || (D % 8 == 0 && freq_rows > 0), "rmsrope_fwd: bad rotary table");
   TT_CHECK(ldx % 8 == 0 && ldy % 8 == 0, "rmsrope_fwd: leading dims misaligned");
   TT_CHECK(aligned16(x) && aligned16(y) && aligned16(w) && aligned16(freqs), "rmsrope_fwd: misaligned pointer");
-  if (C % 256 == 0 && (C <= 2048 || C == 3072 || C == 5120)) {  // one row per warp
+  // A row per warp or per CTA, both measured at 16 to 32,768 rows (us, warp / CTA).  Below about 1,536 rows the warps are too
+  // few to hide the latency of a row that one of them reads alone: 256 rows 9.96 / 3.40 at 3072 per head, 10.6 / 3.5 at
+  // 5120.  Above, the CTA's barriers and idle lanes cost more: 16,384 rows 54.5 / 92.7 at 3072, 80.7 / 104.9 per head, 44.0 /
+  // 86.9 at 2304, 86.0 / 164.1 at 5120.  Rows of 2048 are exactly one vector per thread of a CTA, and with per-head sums,
+  // which need no barrier, it stays ahead: 50.9 against 56.7.  Full rows of up to 2048 go to the warps at any count: the
+  // line is lower there (5.5 / 6.1 at 1536 rows of 1536) and the launches of a Wan block chain (tt_launch).
+  const bool few = rows < 1536;
+  if (C % 256 == 0 && (per_head ? !few && C != 2048 : !few || C <= 2048)) {
     const int want = (rows + NT / 32 - 1) / (NT / 32);
     const int wgrid = want < 148 * 8 ? want : 148 * 8;
 #define TT_RMS_FWD_WARP(NVV)                                                                                              \
@@ -928,8 +934,22 @@ static int rmsrope_fwd_impl(const void* x, long long ldx, void* y, long long ldy
       case 6: TT_RMS_FWD_WARP(6); break;
       case 7: TT_RMS_FWD_WARP(7); break;
       case 8: TT_RMS_FWD_WARP(8); break;
+      case 9: TT_RMS_FWD_WARP(9); break;
+      case 10: TT_RMS_FWD_WARP(10); break;
+      case 11: TT_RMS_FWD_WARP(11); break;
       case 12: TT_RMS_FWD_WARP(12); break;
-      default: TT_RMS_FWD_WARP(20); break;
+      case 13: TT_RMS_FWD_WARP(13); break;
+      case 14: TT_RMS_FWD_WARP(14); break;
+      case 15: TT_RMS_FWD_WARP(15); break;
+      case 16: TT_RMS_FWD_WARP(16); break;
+      case 17: TT_RMS_FWD_WARP(17); break;
+      case 18: TT_RMS_FWD_WARP(18); break;
+      case 19: TT_RMS_FWD_WARP(19); break;
+      case 20: TT_RMS_FWD_WARP(20); break;
+      case 21: TT_RMS_FWD_WARP(21); break;
+      case 22: TT_RMS_FWD_WARP(22); break;
+      case 23: TT_RMS_FWD_WARP(23); break;
+      default: TT_RMS_FWD_WARP(24); break;
     }
 #undef TT_RMS_FWD_WARP
     TT_LAUNCH_CHECK();

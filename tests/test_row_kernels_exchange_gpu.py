@@ -5,6 +5,7 @@ from types import SimpleNamespace
 
 import pytest
 import torch
+from torch.profiler import ProfilerActivity, profile
 
 from teletron_b200.ops import _lib
 from teletron_b200.parallel.fused_ulysses import _scatter_rows
@@ -59,3 +60,23 @@ def test_backward_in_place(C, per_head, rows):
     ref[:, C:2 * C] = dx
     _, dw2 = N.rmsrope_bwd_raw(d[:, C:2 * C], x, w, fr, rstd, 128, per_head, out=d[:, C:2 * C])
     assert torch.equal(d, ref) and torch.equal(dw2, dw)
+
+
+@pytest.mark.parametrize("C", [256, 2048, 2304, 3072, 4096, 5120, 6144])
+@pytest.mark.parametrize("per_head", [False, True])
+@pytest.mark.parametrize("rows", [1535, 1536])
+def test_forward_on_both_sides_of_the_line(C, per_head, rows):
+    """Few rows take a CTA each, many a warp each, which needs their count more than their width."""
+    x, w, fr = _inputs(rows, C, per_head, 400)
+    y, rstd = N.rmsrope_fwd_raw(x, w, fr, 128, per_head)
+    ref = N.rmsnorm_rope_ref(x.float(), w, fr, 128, per_head)
+    heads = x.double().view(rows, -1, 128 if per_head else C)
+    rstd_ref = torch.rsqrt(heads.pow(2).mean(-1) + 1e-6).view(-1)
+    # one bf16 rounding: 1.7e-3 of the norm; fp32 sums
+    assert ((y.float() - ref).norm() / ref.norm()).item() < 2.5e-3
+    torch.testing.assert_close(rstd.double(), rstd_ref, rtol=2e-6, atol=0)
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        N.rmsrope_fwd_raw(x, w, fr, 128, per_head)
+        torch.cuda.synchronize()
+    warp = any("rmsrope_fwd_warp" in e.key for e in prof.key_averages())
+    assert warp == ((rows >= 1536 and C != 2048) if per_head else (rows >= 1536 or C <= 2048))
