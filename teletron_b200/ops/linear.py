@@ -193,6 +193,7 @@ def ffn(x, w1, b1, w2, b2, res, gate=None, rows_per_gate=1, act="gelu"):
 
 _ROWLIN_MAX = 4
 _ROWLIN_CHUNKS = 148
+_PLAIN = (torch.Tensor, torch.nn.Parameter)
 
 
 class _RowLinear(torch.autograd.Function):
@@ -216,29 +217,24 @@ class _RowLinear(torch.autograd.Function):
             return dx, dw, db
         dy = dy.contiguous()
         B, (N, K) = x.shape[0], w.shape
-        L = _lib.lib()
-        dims = (_lib.c_int(B), _lib.c_int(N), _lib.c_int(K))
-        dx = dw = db = None
+        dx = dw = db = partial = None
+        into_main, chunks = False, min(_ROWLIN_CHUNKS, N)
         if ctx.needs_input_grad[0]:
-            chunks = min(_ROWLIN_CHUNKS, N)
             partial = torch.empty((chunks, B, K), dtype=torch.float32, device=x.device)
             dx = torch.empty((B, K), dtype=torch.float32, device=x.device)
-            _lib.check(L.tt_rowlin_dgrad(_lib.ptr(dy), _lib.ptr(w), _lib.ptr(partial), _lib.c_int(chunks), *dims,
-                                         _lib.stream()), "tt_rowlin_dgrad")
-            _lib.check(L.tt_colsum_partials(_lib.ptr(partial), _lib.ptr(dx), _lib.c_int(1), _lib.c_int(chunks),
-                                            _lib.c_int(B * K), _lib.c_int(0), _lib.stream()), "tt_colsum_partials")
         if ctx.needs_input_grad[1]:
-            owner = ctx.w_param
-            mg = main_grad_target(owner)
+            mg = main_grad_target(ctx.w_param)
             into_main = mg is not None and mg.data_ptr() % 16 == 0
             dw = mg if into_main else torch.empty((N, K), dtype=torch.bfloat16, device=x.device)
-            _lib.check(L.tt_rowlin_wgrad(_lib.ptr(dy), _lib.ptr(x), _lib.ptr(dw), _lib.c_int(int(into_main)), *dims,
-                                         _lib.stream()), "tt_rowlin_wgrad")
-            if into_main:
-                dw = None
-                grad_written(owner)
         if ctx.bias_dtype is not None and ctx.needs_input_grad[2]:
-            db = dy.sum(0).to(ctx.bias_dtype)
+            db = torch.empty(N, dtype=torch.bfloat16, device=x.device)
+        _lib.check(_lib.lib().tt_rowlin_bwd(
+            _lib.ptr(dy), _lib.ptr(x), _lib.ptr(w), _lib.ptr(partial), _lib.c_int(chunks), _lib.ptr(dx), _lib.ptr(dw),
+            _lib.c_int(int(into_main)), _lib.ptr(db), _lib.c_int(B), _lib.c_int(N), _lib.c_int(K), _lib.stream()),
+            "tt_rowlin_bwd")
+        if into_main:
+            dw = None
+            grad_written(ctx.w_param)
         return dx, dw, db
 
 
@@ -250,8 +246,7 @@ def row_linear(x, w, b=None):
             and x.shape[1] == w.shape[1] and w.shape[1] % 8 == 0 and w.is_contiguous() and w.data_ptr() % 16 == 0
             and x.device == w.device and w.numel() > 0
             and (b is None or (b.dtype == torch.bfloat16 and b.is_contiguous() and b.shape == w.shape[:1] and b.device == w.device))
-            and all(type(t) in (torch.Tensor, torch.nn.Parameter) for t in (x, w, b) if t is not None)
-            and _lib.plain_call(x.device)):
+            and type(x) in _PLAIN and type(w) in _PLAIN and (b is None or type(b) in _PLAIN) and _lib.plain_call(x.device)):
         x = x.float().contiguous()
         if x.data_ptr() % 16:          # a slice at an odd offset
             x = x.clone()
