@@ -109,8 +109,8 @@ class T5SelfAttentionBlock(nn.Module):
         return x + self.ffn(self.norm2(x))
 
 
-_MODULES = (T5SelfAttentionBlock, T5LayerNorm, T5Attention, T5RelativeEmbedding, T5FeedForward, nn.Embedding, nn.Linear,
-            nn.GELU, nn.ModuleList, nn.Sequential)
+_MODULES = frozenset((T5SelfAttentionBlock, T5LayerNorm, T5Attention, T5RelativeEmbedding, T5FeedForward, nn.Embedding,
+                      nn.Linear, nn.GELU, nn.ModuleList, nn.Sequential))
 
 
 class UMT5Encoder(nn.Module):
@@ -134,10 +134,13 @@ class UMT5Encoder(nn.Module):
             return False
         if mask is not None and (mask.shape != ids.shape or mask.device != ids.device):
             return False
-        if not plain_call(ids.device) or type(ids) is not torch.Tensor or not plain_modules(self, _MODULES, root_hooks=False):
+        if not plain_call(ids.device) or type(ids) is not torch.Tensor:
+            return False
+        mods = plain_modules(self, _MODULES, root_hooks=False)
+        if mods is None:
             return False
         grad = torch.is_grad_enabled()
-        for m in self.modules():
+        for m in mods:
             for p in m._parameters.values():
                 if p is not None and (p.dtype != torch.bfloat16 or p.device != ids.device or not p.is_contiguous()
                                       or (grad and p.requires_grad) or p.data_ptr() % 16):

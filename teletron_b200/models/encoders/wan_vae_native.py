@@ -17,8 +17,8 @@ from ..native_route import plain_modules
 from . import wan_vae as V
 
 
-_MODULES = (V.CausalConv3d, V.RMS_norm, V.Resample, V.ResidualBlock, V.AttentionBlock, nn.Conv2d, nn.SiLU, nn.Dropout,
-            nn.Identity, nn.Upsample, nn.ZeroPad2d, nn.Sequential)
+_MODULES = frozenset((V.CausalConv3d, V.RMS_norm, V.Resample, V.ResidualBlock, V.AttentionBlock, nn.Conv2d, nn.SiLU, nn.Dropout,
+                      nn.Identity, nn.Upsample, nn.ZeroPad2d, nn.Sequential))
 
 
 def usable(net: nn.Module, x: torch.Tensor) -> bool:
@@ -33,13 +33,16 @@ def usable(net: nn.Module, x: torch.Tensor) -> bool:
             return False
     elif x.dtype != torch.bfloat16:
         return False
-    if not plain_call(x.device) or type(x) is not torch.Tensor or not plain_modules(net, _MODULES):
+    if not plain_call(x.device) or type(x) is not torch.Tensor:
+        return False
+    mods = plain_modules(net, _MODULES)
+    if mods is None:
         return False
     grad = torch.is_grad_enabled()
     if grad and x.requires_grad:
         return False
     first, last = net.conv1, net.head[2]
-    for m in net.modules():
+    for m in mods:
         if isinstance(m, nn.Dropout) and m.training and m.p > 0:
             return False
         if isinstance(m, (nn.Conv2d, nn.Conv3d)):

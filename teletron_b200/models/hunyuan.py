@@ -416,7 +416,6 @@ class SingleStreamBlock(nn.Module):
         xt = _project_out(self.proj_out, ct, xt, e[:, 2], rt)
         return xv, xt
 
-
     def packed_infer(self, x, n_video, temb, freqs, text_lens):
         """The block on one sample's rows [video | text] without splitting them: the two streams share every weight, so
         norm, projections and attention take the packed rows, the attention output and the MLP's hidden rows are
@@ -453,8 +452,11 @@ class SingleStreamBlock(nn.Module):
             return False
         if x.dtype != torch.bfloat16 or self.proj_mlp.bias is None or self.proj_out.weight.shape[1] != C + self.proj_mlp.weight.shape[0]:
             return False
-        return plain_modules(self, (HunyuanAttention, FusedColumnParallel, HeadNorm, AdaNormZero, ColumnParallelLinear,
-                                    SingleProjOut, nn.Linear))
+        return plain_modules(self, _SINGLE_MODULES) is not None
+
+
+_SINGLE_MODULES = frozenset((HunyuanAttention, FusedColumnParallel, HeadNorm, AdaNormZero, ColumnParallelLinear, SingleProjOut,
+                             nn.Linear))
 
 
 class _PairBlock(nn.Module):

@@ -292,7 +292,8 @@ def _block_params(blk: DiTBlock):
             ca.norm_k.weight, ca.o.weight, ca.o.bias, f1.weight, f1.bias, f2.weight, f2.bias)
 
 
-_BLOCK_MODULES = (SelfAttention, CrossAttention, FusedProj, RMSNormWeight, nn.Linear, nn.LayerNorm, nn.GELU, nn.Sequential)
+_BLOCK_MODULES = frozenset((SelfAttention, CrossAttention, FusedProj, RMSNormWeight, nn.Linear, nn.LayerNorm, nn.GELU,
+                            nn.Sequential))
 
 
 def wan_block_infer(blk: DiTBlock, x2d, context, t_mod, freqs, batch: int, cp):
@@ -305,7 +306,7 @@ def wan_block_infer(blk: DiTBlock, x2d, context, t_mod, freqs, batch: int, cp):
         return None
     if any(type(t) is not torch.Tensor for t in (x2d, context, t_mod, freqs)):
         return None
-    if not plain_modules(blk, _BLOCK_MODULES, root_hooks=False) or not blk.eps == blk.self_attn.eps == blk.cross_attn.eps:
+    if plain_modules(blk, _BLOCK_MODULES, root_hooks=False) is None or not blk.eps == blk.self_attn.eps == blk.cross_attn.eps:
         return None
     bf16 = torch.bfloat16
     C, dev, (B, Lc, Cc) = blk.dim, x2d.device, context.shape

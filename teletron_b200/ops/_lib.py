@@ -14,6 +14,9 @@ from pathlib import Path
 
 import torch
 
+_is_tracing, _dispatch_modes = torch._C._is_tracing, torch._C._len_torch_dispatch_stack
+_functorch_level, _forward_ad = torch._C._functorch.peek_interpreter_stack, torch.autograd.forward_ad
+
 _LOCK = threading.Lock()
 _LIB = None
 _STATUS: dict[int, torch.Tensor] = {}
@@ -124,9 +127,8 @@ def plain_call(device: torch.device) -> bool:
     compiling, forward-mode AD, functorch transforms, dispatch modes)."""
     if device.type != "cuda" or device.index != torch.cuda.current_device():
         return False
-    return not (torch.is_autocast_enabled("cuda") or torch.jit.is_tracing() or torch.compiler.is_compiling()
-                or torch.autograd.forward_ad._current_level >= 0
-                or torch._C._functorch.peek_interpreter_stack() is not None or torch._C._len_torch_dispatch_stack())
+    return not (torch.is_autocast_enabled("cuda") or _is_tracing() or torch.compiler.is_compiling()
+                or _forward_ad._current_level >= 0 or _functorch_level() is not None or _dispatch_modes())
 
 
 def main_grad_of(p):
@@ -135,23 +137,29 @@ def main_grad_of(p):
     return mg if mg is not None and mg.dtype == torch.float32 and mg.is_contiguous() else None
 
 
-def main_grad_target(p):
+def main_grad_target(p, edge):
     """``main_grad_of(p)`` when the backward pass in progress may add p's gradient there and return None for it, else
     None.  It may not when somebody is to see the gradient: ``autograd.grad`` hands it out, ``backward(inputs=...)`` may
     leave p out, tensor hooks and post-accumulate hooks (other than the optimizer's) read it.  Autograd runs p's
     AccumulateGrad once all uses of p in the pass are done, also when their gradients are undefined, so the
-    optimizer learns there that p's gradient is complete (parallel/ddp.py)."""
+    optimizer learns there that p's gradient is complete (parallel/ddp.py).  ``edge``: the entry of the calling node's
+    ``next_functions`` that leads to p, directly or through a conversion and a reshape."""
     mg = main_grad_of(p)
     if mg is None or p._backward_hooks:
         return None
     hooks = p._post_accumulate_grad_hooks
     if hooks and len(hooks) > int(hasattr(p, "grad_ready")):
         return None
+    node = edge[0]
+    for _ in range(2):
+        if node is not None and not hasattr(node, "variable"):
+            node = node.next_functions[0][0] if node.next_functions else None
+    if getattr(node, "variable", None) is not p:
+        return None
     try:
-        runs = torch._C._will_engine_execute_node(torch.autograd.graph.get_gradient_edge(p).node)
+        return mg if torch._C._will_engine_execute_node(node) else None
     except RuntimeError:      # autograd.grad with p among its inputs
         return None
-    return mg if runs else None
 
 
 def grad_written(p) -> None:

@@ -169,10 +169,11 @@ class _SelfAttnCore(torch.autograd.Function):
         v4 = qkv[:, 2 * C:3 * C].unflatten(1, (H, D)).unflatten(0, (batch, S))
         attention_bwd(q.view(batch, S, H, D), k.view(batch, S, H, D), v4, o, lse, do.view(batch, S, H, D),
                       out=(dqn, dkn, dv_view))
+        owners = [None if p is None else (p, edge) for p, edge in zip(ctx.owners, ctx.next_functions[1:3])]
         _, dwq = rmsrope_bwd_raw(dqn.view(batch * S, C), qkv[:, 0:C], wqf, freqs, rq, D, False, out=dqkv[:, 0:C],
-                                 owner=ctx.owners[0])
+                                 owner=owners[0])
         _, dwk = rmsrope_bwd_raw(dkn.view(batch * S, C), qkv[:, C:2 * C], wkf, freqs, rk, D, False,
-                                 out=dqkv[:, C:2 * C], owner=ctx.owners[1])
+                                 out=dqkv[:, C:2 * C], owner=owners[1])
         dwq, dwk = (None if g is None else g.to(wdtype) for g in (dwq, dwk))
         return dqkv, dwq, dwk, None, None, None, None, None, None
 

@@ -73,12 +73,12 @@ def _weight_grad(dy, x, w, owner=None):
     return gemm(dy, x, a_mn=True, b_mn=True, out_dtype=w.dtype)
 
 
-def _bias_grad(dy, b):
+def _bias_grad(dy, b, edge):
     """Column sums of dy: added to the parameter's fp32 gradient buffer where that may take it (returns None: no bf16
     copy, no accumulation in bf16 over micro-batches, no fold afterwards), else a gradient of the bias' type."""
     if b is None:
         return None
-    mg = main_grad_target(b) if dy.is_cuda else None
+    mg = main_grad_target(b, edge) if dy.is_cuda else None
     if mg is not None and mg.numel() == dy.shape[1]:
         colsum(dy, add_to=mg.view(-1))
         grad_written(b)
@@ -110,7 +110,7 @@ class _Linear(torch.autograd.Function):
             dy = act_bwd(dy, pre, ctx.act)
         dx = gemm(dy, w, b_mn=True) if ctx.needs_input_grad[0] else None
         dw = _weight_grad(dy, x, w, ctx.w_param) if ctx.needs_input_grad[1] else None
-        db = _bias_grad(dy, ctx.bias_ref) if (ctx.has_bias and ctx.needs_input_grad[2]) else None
+        db = _bias_grad(dy, ctx.bias_ref, ctx.next_functions[2]) if (ctx.has_bias and ctx.needs_input_grad[2]) else None
         return dx, dw, db, None
 
 
@@ -169,7 +169,7 @@ class _LinearResidual(torch.autograd.Function):
             dz = dy
         dx = gemm(dz, w, b_mn=True) if ctx.needs_input_grad[0] else None
         dw = _weight_grad(dz, x, w, ctx.w_param) if ctx.needs_input_grad[1] else None
-        db = _bias_grad(dz, b) if (b is not None and ctx.needs_input_grad[2]) else None
+        db = _bias_grad(dz, b, ctx.next_functions[2]) if (b is not None and ctx.needs_input_grad[2]) else None
         dres = dy if ctx.needs_input_grad[3] else None
         return dx, dw, db, dres, dgate, None
 
@@ -223,7 +223,7 @@ class _RowLinear(torch.autograd.Function):
             partial = torch.empty((chunks, B, K), dtype=torch.float32, device=x.device)
             dx = torch.empty((B, K), dtype=torch.float32, device=x.device)
         if ctx.needs_input_grad[1]:
-            mg = main_grad_target(ctx.w_param)
+            mg = main_grad_target(ctx.w_param, ctx.next_functions[1])
             into_main = mg is not None and mg.data_ptr() % 16 == 0
             dw = mg if into_main else torch.empty((N, K), dtype=torch.bfloat16, device=x.device)
         if ctx.bias_dtype is not None and ctx.needs_input_grad[2]:

@@ -84,7 +84,7 @@ class _AdaLN(torch.autograd.Function):
         if dres is not None and (dres.dtype != torch.bfloat16 or dres.stride(1) != 1):
             dres = dres.to(torch.bfloat16).contiguous()
         dx = torch.empty((rows, C), dtype=torch.bfloat16, device=x.device)
-        targets = None if ctx.owners is None else tuple(_lib.main_grad_target(p) for p in ctx.owners)
+        targets = None if ctx.owners is None else tuple(map(_lib.main_grad_target, ctx.owners, ctx.next_functions[1:3]))
         into_main = targets is not None and None not in targets
         want_mod = (scale is not None and ctx.needs_input_grad[1]) or (has_shift and ctx.needs_input_grad[2])
         chunks = _chunks(rows_per_batch, batch)
@@ -205,14 +205,15 @@ class _RmsRope(torch.autograd.Function):
     def backward(ctx, dy):
         x, wf, freqs, rstd = ctx.saved_tensors
         D, per_head, wdtype = ctx.meta
-        dx, dw = rmsrope_bwd_raw(dy, x, wf, freqs, rstd, D, per_head, owner=ctx.owner)
+        owner = (ctx.owner, ctx.next_functions[1]) if ctx.owner is not None else None
+        dx, dw = rmsrope_bwd_raw(dy, x, wf, freqs, rstd, D, per_head, owner=owner)
         return dx, (dw.to(wdtype) if dw is not None else None), None, None, None, None
 
 
 def rmsrope_bwd_raw(dy, x, wf, freqs, rstd, D, per_head=False, out=None, owner=None):
     """Backward of rope(rmsnorm(x) * w) from the saved input and rstd: returns (dx bf16, dw fp32 or None).
-    ``out``: optional [rows, C] view (any row stride) that receives dx.  ``owner``: the weight parameter; a full-row
-    weight gradient is added to its fp32 buffer where that may take it (dw is None then)."""
+    ``out``: optional [rows, C] view (any row stride) that receives dx.  ``owner``: the weight parameter and the calling
+    node's edge to it; a full-row weight gradient is added to its fp32 buffer where that may take it (dw is None then)."""
     rows, C = x.shape
     if dy.stride(1) != 1:
         dy = dy.contiguous()
@@ -231,13 +232,13 @@ def rmsrope_bwd_raw(dy, x, wf, freqs, rstd, D, per_head=False, out=None, owner=N
     _lib.check(rc, "tt_rmsrope_bwd")
     dw = None
     if wf is not None:
-        mg = None if owner is None or per_head else _lib.main_grad_target(owner)
+        mg = None if owner is None or per_head else _lib.main_grad_target(*owner)
         dwf = torch.empty((1, C), dtype=torch.float32, device=x.device) if mg is None else mg
         rc = L.tt_colsum_partials(_lib.ptr(partial), _lib.ptr(dwf), _lib.c_int(1), _lib.c_int(ctas),
                                   _lib.c_int(C), _lib.c_int(int(mg is not None)), _lib.stream())
         _lib.check(rc, "tt_colsum_partials")
         if mg is not None:
-            _lib.grad_written(owner)
+            _lib.grad_written(owner[0])
             return dx, None
         dw = dwf.view(C // D, D).sum(0) if per_head else dwf.view(C)
     return dx, dw

@@ -279,7 +279,9 @@ class _FusedUlyssesFn(torch.autograd.Function):
         _, dwk = rmsrope_bwd_raw(dqkv[:, C:2 * C], k_pre, wk_f, freqs, rstd_k, D, False, out=dqkv[:, C:2 * C])
         dx = gemm(dqkv, w_qkv, b_mn=True) if ctx.needs_input_grad[1] else None
         dw = _weight_grad(dqkv, x, w_qkv, ctx.w_param) if ctx.needs_input_grad[2] else None
-        db = _bias_grad(dqkv, ctx.bias_ref) if (ctx.bias_ref is not None and ctx.needs_input_grad[3]) else None
+        db = None
+        if ctx.bias_ref is not None and ctx.needs_input_grad[3]:
+            db = _bias_grad(dqkv, ctx.bias_ref, ctx.next_functions[2])   # the tensors: x, the weight, the bias
         # layers run backward in reverse order, so this layer's region is the top of the stack
         if fu.slab.live and fu.slab.live[-1][1] == fu.slab.off:
             fu.slab.release_to(fu.slab.live.pop()[0])

@@ -201,7 +201,7 @@ class _FusedColumnLinear(torch.autograd.Function):
         if ctx.needs_input_grad[1]:
             xg = x_rows if ctx.have_gathered else _ag_rows(x_rows, tp.group, tp.size)
             dw = _weight_grad(dy, xg, w, ctx.w_param)
-        db = _bias_grad(dy, ctx.bias_ref) if (ctx.bias_ref is not None and ctx.needs_input_grad[2]) else None
+        db = _bias_grad(dy, ctx.bias_ref, ctx.next_functions[2]) if (ctx.bias_ref is not None and ctx.needs_input_grad[2]) else None
         return dx, dw, db, None, None
 
 

@@ -19,7 +19,7 @@ def _shared_vector_worker(rank, world):
 
         @staticmethod
         def backward(ctx, dy):
-            mg, dv = _lib.main_grad_target(ctx.v), dy.sum(0)
+            mg, dv = _lib.main_grad_target(ctx.v, ctx.next_functions[1]), dy.sum(0)
             if mg is None:
                 return dy, dv
             assert not fired()
