@@ -246,7 +246,7 @@ TT_API int tt_gemm_bf16(const void* A, long long lda, int a_mn, const void* B, l
   int dev = 0, sms = 0;
   TT_CUDA(cudaGetDevice(&dev));
   TT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  const int split = (max_ctas <= 0 && N > 64) ? splitk_factor(M, N, K, sms) : 1;
+  const int split = (max_ctas <= 0 && N > 64) ? splitk_factor(M, N, K, sms, 16) : 1;
   const int BN = split > 1 ? 128 : N > 128 ? 256 : (N > 64 ? 128 : 64);
   CUtensorMap tmA, tmB;
   {

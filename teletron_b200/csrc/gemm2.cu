@@ -360,7 +360,7 @@ TT_API int tt_gemm2_bf16(const void* A, long long lda, int a_mn, const void* B, 
   int dev = 0, sms = 0;
   TT_CUDA(cudaGetDevice(&dev));
   TT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  const int split = splitk_factor(M, N, K, sms);
+  const int split = splitk_factor(M, N, K, sms, 8);
   if (split > 1) return tt_gemm_splitk(tmA, tmB, a_mn, b_mn, p, split, stream);  // the maps have the same boxes
   if (!a_mn && !b_mn) return launch2<0, 0>(tmA, tmB, p, sms, stream);
   if (!a_mn && b_mn) return launch2<0, 1>(tmA, tmB, p, sms, stream);

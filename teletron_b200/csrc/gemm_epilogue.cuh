@@ -247,13 +247,22 @@ __device__ __forceinline__ void epilogue_tile_qkv(const GemmParams& p, uint32_t 
   }
 }
 
+// how many clusters of 2, 4 or 8 split-K CTAs the current device holds at a time (a cluster sits in one GPC, so this is
+// less than the SMs over the cluster's size)
+int splitk_clusters(int split);
+
 // Products whose 128 x 128 output tiles would leave half of the SMs idle are cut along K (csrc/gemm_splitk.cu): by how
-// much, or 1.  Each part keeps at least four 64-wide steps, below that the start-up of a CTA outweighs its loop.
-inline int splitk_factor(int M, int N, int K, int sms) {
+// much, or 1.
+//   - All clusters run at once: 16 tiles x 8 parts need a second wave for a few of them (512 x 512 x 5120: 25.0 us, 1,024 x
+//     512 with 32 tiles x 4 15.2), and so do 36 x 4 (2,304 x 256 x 1024: 17.7 us, whole 14.1).
+//   - Each part keeps at least four 64-wide steps, below that the start-up of a CTA outweighs its loop.
+//   - Against the one-CTA kernel, which starts faster than the pair kernel, K has to be at least 1,024 (min_steps = 16): 128 x
+//     128 x 512 takes 6.5 us whole and 8.6 in two parts, 256 x 512 x 512 10.7 by the pair kernel and 8.7 in two parts.
+inline int splitk_factor(int M, int N, int K, int sms, int min_steps) {
   const long long tiles = (long long)((M + 127) / 128) * ((N + 127) / 128);
   const int num_kb = (K + BK - 1) / BK;
   int s = 1;
-  while (s < 8 && tiles * s * 2 <= sms && num_kb >= 8 * s) s *= 2;
+  while (s < 8 && tiles * s * 2 <= sms && num_kb >= 8 * s && num_kb >= min_steps && tiles <= splitk_clusters(2 * s)) s *= 2;
   return s;
 }
 

@@ -8,7 +8,10 @@
 // workspace, no atomics: the result does not depend on timing.
 //
 // Roles (320 threads): warp 0 TMA producer, warp 1 tensor memory + MMA issue, warps 2..9 drain the accumulator, all
-// threads add up.  Every wait is bounded.
+// threads add up.  Every mbarrier wait is bounded.  The two cluster barriers are reached by every thread of every CTA:
+// no role returns early, and one whose wait ran out goes on to them with the abort flag set.
+#include <atomic>
+
 #include "gemm_epilogue.cuh"
 
 using namespace tt;
@@ -173,6 +176,34 @@ int launch_splitk(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmPara
 }
 
 }  // namespace
+
+int tt_gemm::splitk_clusters(int split) {
+  constexpr int DEVS = 16;
+  static std::atomic<int> known[DEVS][4];  // a property of the device and the kernel; 0: not asked yet
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev >= DEVS) return 0;
+  std::atomic<int>& slot = known[dev][split == 2 ? 1 : split == 4 ? 2 : 3];
+  if ((n = slot.load(std::memory_order_relaxed)) == 0) {
+    auto kern = gemm_splitk_kernel<0, 0>;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = split;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.gridDim = dim3(split);
+    cfg.blockDim = dim3(320);
+    cfg.dynamicSmemBytes = SK_SMEM;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SK_SMEM) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      return 0;
+    }
+    slot.store(n, std::memory_order_relaxed);
+  }
+  return n;
+}
 
 int tt_gemm_splitk(const CUtensorMap& tmA, const CUtensorMap& tmB, int a_mn, int b_mn, const GemmParams& p, int split,
                    cudaStream_t stream) {

@@ -50,9 +50,10 @@ def _kernels(fn):
     return out, " ".join(e.key for e in prof.key_averages())
 
 
-# the largest number of 128 x 128 tiles that is split on 148 SMs is 74; K in steps of 64, at least eight of them
-@pytest.mark.parametrize("M,N,K,split", [(256, 1536, 8960, True), (128, 136, 512, True), (2304, 512, 512, True),
-                                         (2432, 512, 512, False), (128, 136, 448, False), (256, 64, 2048, False)])
+# on 148 SMs: at most 74 tiles of 128 x 128; K of at least 512 from the pair kernel (256 x 256 outputs), 1,024 from the other
+@pytest.mark.parametrize("M,N,K,split", [(256, 1536, 8960, True), (128, 136, 1024, True), (2176, 512, 512, True),
+                                         (2432, 512, 512, False), (128, 136, 960, False), (256, 264, 448, False),
+                                         (512, 512, 5120, True), (256, 64, 2048, False)])
 @pytest.mark.parametrize("form", ["null gate", "fp32", "fp32 accumulate"])
 def test_splitk_forms(M, N, K, split, form):
     torch.manual_seed(1)
