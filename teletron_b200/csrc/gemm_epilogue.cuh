@@ -165,6 +165,7 @@ __device__ __forceinline__ void epilogue_tile(const GemmParams& p, uint32_t acc,
   const float* gate_row = nullptr;
   if (p.epi == EPI_GATE_RES && p.gate && row_ok)
     gate_row = p.gate + (long long)(row / p.rows_per_gate) * p.gate_ld;
+  if (!__any_sync(0xffffffffu, row_ok)) return;  // 64 rows or fewer leave half of the warps nothing to do
 #pragma unroll 1
   for (int c = eg * (BN / 64); c < (eg + 1) * (BN / 64); ++c) {
     uint32_t r[32];
