@@ -232,9 +232,10 @@ adaln_fwd_warp_kernel(const bf16* __restrict__ x, long long ldx, bf16* __restric
 // ------------------------------------------------------------------ AdaLN backward
 // grid = (chunks, batch). CTA (chunk, b) owns rows [b*rpb + chunk*rpc, min(.. + rpc, (b+1)*rpb)).
 // A CTA walks its rows one after the other, so what bounds it is the latency of a row: the next row's loads are issued
-// before this row's reduction, the reduction buffer alternates (one barrier per row), and rows stay packed (the values
-// are unpacked again for the second pass) so that two or more CTAs fit an SM.
-template <int VPT, int NTH, int MINB>
+// before this row's reduction (AHEAD), and the reduction buffer alternates (one barrier per row).  With one vector per
+// thread the first pass' values are kept for the second (KEEP); with two, rows stay packed and are unpacked again, so
+// that two CTAs fit an SM.
+template <int VPT, int NTH, int MINB, bool AHEAD, bool KEEP>
 __global__ void __launch_bounds__(NTH, MINB)
 adaln_bwd_kernel(const bf16* __restrict__ dy, long long lddy, const bf16* __restrict__ x,
                  long long ldx, const float* __restrict__ mean_in, const float* __restrict__ rstd_in,
@@ -266,7 +267,7 @@ adaln_bwd_kernel(const bf16* __restrict__ dy, long long lddy, const bf16* __rest
     nmean = mean_in[row];
     nrstd = rstd_in[row];
   };
-  if (r0 < r1) fetch(r0);
+  if (AHEAD && r0 < r1) fetch(r0);
 #pragma unroll
   for (int k = 0; k < VPT; ++k) {
     const int vec = threadIdx.x + k * NTH;
@@ -285,7 +286,19 @@ adaln_bwd_kernel(const bf16* __restrict__ dy, long long lddy, const bf16* __rest
   for (int r = r0; r < r1; ++r) {
     const long long row = (long long)b * rows_per_batch + r;
     uint4 cd[VPT], cx[VPT], ce[VPT];
+    float g[VPT][8], xh[VPT][8];
+    if (!AHEAD) fetch(r);
     const float mean = nmean, rstd = nrstd;
+    auto unpack = [&](int k, float (&d)[8]) {
+      float xv[8];
+      unpack8(cd[k], d);
+      unpack8(cx[k], xv);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        xh[k][j] = (xv[j] - mean) * rstd;
+        g[k][j] = d[j] * m[k][j];
+      }
+    };
 #pragma unroll
     for (int k = 0; k < VPT; ++k) {
       cd[k] = nd[k];
@@ -294,21 +307,19 @@ adaln_bwd_kernel(const bf16* __restrict__ dy, long long lddy, const bf16* __rest
       ce[k] = make_uint4(0, 0, 0, 0);
       if (dx_add && vec < nvec) ce[k] = ldraw(dx_add + row * ldadd + vec * 8);
     }
-    if (r + 1 < r1) fetch(r + 1);
+    if (AHEAD && r + 1 < r1) fetch(r + 1);
     float2 s = make_float2(0.f, 0.f);
 #pragma unroll
     for (int k = 0; k < VPT; ++k) {
       if (threadIdx.x + k * NTH < nvec) {
-        float d[8], xv[8];
-        unpack8(cd[k], d);
-        unpack8(cx[k], xv);
+        float d[8];
+        unpack(k, d);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-          const float xh = (xv[j] - mean) * rstd, g = d[j] * m[k][j];
-          acc_mul[k][j] += d[j] * xh;
+          acc_mul[k][j] += d[j] * xh[k][j];
           acc_add[k][j] += d[j];
-          s.x += g;
-          s.y += g * xh;
+          s.x += g[k][j];
+          s.y += g[k][j] * xh[k][j];
         }
       }
     }
@@ -328,14 +339,16 @@ adaln_bwd_kernel(const bf16* __restrict__ dy, long long lddy, const bf16* __rest
     for (int k = 0; k < VPT; ++k) {
       const int vec = threadIdx.x + k * NTH;
       if (vec < nvec) {
-        float d[8], xv[8], e[8], o[8];
-        forget(cd[k]);
-        forget(cx[k]);
-        unpack8(cd[k], d);
-        unpack8(cx[k], xv);
+        float e[8], o[8];
+        if (!KEEP) {
+          float d[8];
+          forget(cd[k]);
+          forget(cx[k]);
+          unpack(k, d);
+        }
         unpack8(ce[k], e);  // the residual-branch gradient, zero without one
 #pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] = rstd * (d[j] * m[k][j] - c1 - (xv[j] - mean) * rstd * c2) + e[j];
+        for (int j = 0; j < 8; ++j) o[j] = rstd * (g[k][j] - c1 - xh[k][j] * c2) + e[j];
         store8(dx + row * lddx + vec * 8, o);
       }
     }
@@ -566,16 +579,21 @@ TT_API int tt_adaln_bwd(const void* dy, long long lddy, const void* x, long long
            "adaln_bwd: misaligned pointer");
   const int rpc = (rows_per_batch + chunks - 1) / chunks;
   dim3 grid(chunks, batch);
-#define TT_ADALN_BWD(V, T, B)                                                                                           \
-  adaln_bwd_kernel<V, T, B><<<grid, T, 0, stream>>>((const bf16*)dy, lddy, (const bf16*)x, ldx, mean, rstd, mul, mod_ld, \
-                                                    plus_one, (bf16*)dx, lddx, (const bf16*)dx_add, ldadd, partial, C,   \
-                                                    rows_per_batch, rpc)
-  // few idle lanes at the usual widths (1536, 2048, 3072, 5120) and at most two vectors per thread
-  if (C <= 1536) TT_ADALN_BWD(1, 192, 5);
-  else if (C <= 2048) TT_ADALN_BWD(1, 256, 4);
-  else if (C <= 3072) TT_ADALN_BWD(1, 384, 2);
-  else if (C <= 5120) TT_ADALN_BWD(2, 320, 2);
-  else TT_ADALN_BWD(2, 384, 1);
+#define TT_ADALN_BWD(V, T, ...)                                                                                        \
+  adaln_bwd_kernel<V, T, __VA_ARGS__><<<grid, T, 0, stream>>>((const bf16*)dy, lddy, (const bf16*)x, ldx, mean, rstd, mul, \
+                                                              mod_ld, plus_one, (bf16*)dx, lddx, (const bf16*)dx_add,   \
+                                                              ldadd, partial, C, rows_per_batch, rpc)
+  // Few idle lanes and at most two vectors per thread; up to 2048 columns the 592 CTAs that callers ask for are resident at
+  // once (four per SM).  us at 4,096 / 32,760 rows, in brackets by CTAs of 256 threads for every width, two barriers per row
+  // and nothing in flight:
+  //   1024: 24.6 / 71.8 (25.4 / 92.8)   1536: 28.3 / 91.1 (27.2 / 104.7)   2048: 31.2 / 116.1 (30.6 / 118.7)
+  // At 2048 the registers of four CTAs do not hold the next row beside the kept values (40.1 / 178 with it).
+  if (C <= 1024) TT_ADALN_BWD(1, 128, 5, true, true);
+  else if (C <= 1536) TT_ADALN_BWD(1, 192, 4, true, true);
+  else if (C <= 2048) TT_ADALN_BWD(1, 256, 4, false, true);
+  else if (C <= 3072) TT_ADALN_BWD(1, 384, 2, true, false);
+  else if (C <= 5120) TT_ADALN_BWD(2, 320, 2, true, false);
+  else TT_ADALN_BWD(2, 384, 1, true, false);
 #undef TT_ADALN_BWD
   TT_LAUNCH_CHECK();
   if (partial && (dmul || dadd)) {

@@ -80,3 +80,21 @@ def test_forward_on_both_sides_of_the_line(C, per_head, rows):
         torch.cuda.synchronize()
     warp = any("rmsrope_fwd_warp" in e.key for e in prof.key_averages())
     assert warp == ((rows >= 1536 and C != 2048) if per_head else (rows >= 1536 or C <= 2048))
+
+
+@pytest.mark.parametrize("C", [8, 1024, 1032, 1536, 1544, 2048, 2056])
+@pytest.mark.parametrize("rows,residual", [(1, True), (5, False), (1300, True)])
+def test_adaln_backward_on_both_sides_of_the_lines(C, rows, residual):
+    """Widths around each change of the number of threads and of what is kept in registers."""
+    torch.manual_seed(2)
+    x, dy, dr = (torch.randn(rows, C, device="cuda", dtype=BF16) for _ in range(3))
+    e = torch.randn(1, 2, C, device="cuda")
+    xg, eg = x.clone().requires_grad_(), e.clone().requires_grad_()
+    y, xr = N.adaln_res(xg, eg[:, 1], eg[:, 0], rows)
+    dx, de = torch.autograd.grad([y, xr] if residual else [y], [xg, eg], [dy, dr] if residual else [dy])
+    xd, ed = x.double().requires_grad_(), e.double().requires_grad_()
+    yd = torch.nn.functional.layer_norm(xd, (C,), eps=1e-6) * (1 + ed[:, 1]) + ed[:, 0]
+    dxd, ded = torch.autograd.grad([yd, xd * 1.0] if residual else [yd], [xd, ed], [dy.double(), dr.double()] if residual else [dy.double()])
+    # one bf16 rounding of the output (1.7e-3 of the norm, at most 2^-8); the column sums stay in fp32
+    assert ((dx.double() - dxd).norm() / dxd.norm()).item() < (2.5e-3 if rows * C > 1000 else 2 ** -8)
+    assert ((de.double() - ded).norm() / ded.norm()).item() < 1e-5
