@@ -110,8 +110,10 @@ TT_API int tt_wan_block_fwd(const void* x, long long ldx, void* out, const void*
   pp.mod = par(P_MOD); pp.t_mod = t_mod; pp.out = w.small; pp.B = B; pp.C = C;
   const int rows6[6] = {P_NQ, P_NK, P_N3_W, P_N3_B, P_CNQ, P_CNK};
   for (int i = 0; i < 6; ++i) pp.rows[i] = par(rows6[i]);
-  // start-ups overlapped with the launch before: 12.4 -> 11.2 ms for a step of 256 tokens, 549.8 -> 552.7 ms for one of
-  // 32,760, whose kernels are too long for it to matter
+  // Start-ups overlapped with the launch before.  A forward pass of eight 1536-wide blocks, without -> with, ms:
+  //   256 tokens 1.76 -> 1.59, 1,024 2.54 -> 2.39, 3,072 3.49 -> 3.34, 6,144 6.71 -> 6.39;
+  //   8,192 9.93 -> 9.98, 12,288 16.30 -> 16.35, 16,384 25.39 -> 25.56, 24,576 44.80 -> 45.02
+  // so the line lies where it stops paying.  5120-wide blocks: within noise on both sides of it (+-3 %).
   const TTChain chain(R < 8192);
   TT_CUDA(tt_launch(wan_prep_kernel, dim3((C + 255) / 256, 6 * B + 6), dim3(256), 0, stream, 1, pp));
   TT_LAUNCH_CHECK();
